@@ -3,7 +3,7 @@
 // One CTA computes one output tile C[m0:m0+BM, n0:n0+BN] of a column-major
 // M x N matrix as the sum, over its K-segments, of A_s(M x K_s) * B_s(K_s x N)
 // with both operands column-major (A M-contiguous, B K-contiguous).  Tiles of
-// ragged size are handled by zero-filled copies.
+// ragged size cost their size rounded up to 8 x 8 blocks (tile_dmma.cuh).
 //
 // Arithmetic: FP64 tensor-core MMA (mma.sync m8n8k4 .f64), the FP64 tensor
 // pipe of sm_100a (tcgen05 has no FP64 kind).  Operands are staged

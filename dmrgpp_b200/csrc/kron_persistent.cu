@@ -50,7 +50,7 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
 
 template <class C>
 __device__ __forceinline__ void
-store_tile(const tile::Acc<C>& acc, double* Cp, int ldc, int m0, int n0, int M, int N)
+store_tile(const tile::Acc<C>& acc, double* Cp, int ldc, int m0, int n0, int M, int N, int slot)
 {
 #pragma unroll
 	for (int mi = 0; mi < C::MI; ++mi)
@@ -58,15 +58,15 @@ store_tile(const tile::Acc<C>& acc, double* Cp, int ldc, int m0, int n0, int M, 
 		for (int ni = 0; ni < C::NI; ++ni)
 #pragma unroll
 			for (int h = 0; h < 2; ++h) {
-				const int row = m0 + tile::acc_row<C>(mi);
-				const int col = n0 + tile::acc_col<C>(ni, h);
+				const int row = m0 + tile::acc_row<C>(slot, mi);
+				const int col = n0 + tile::acc_col<C>(slot, ni, h);
 				if (row < M && col < N)
 					Cp[(long long)col * ldc + row] = acc.v[mi][ni][h];
 			}
 }
 
 template <class C>
-__global__ void __launch_bounds__(C::THREADS) kron_persistent_kernel(PersistentArgs a)
+__global__ void __launch_bounds__(C::THREADS, C::CTAS) kron_persistent_kernel(PersistentArgs a)
 {
 	extern __shared__ __align__(16) double smem[];
 	__shared__ __align__(16) KronItem s_w[2];
@@ -137,12 +137,44 @@ __global__ void __launch_bounds__(C::THREADS) kron_persistent_kernel(PersistentA
 		const KronItem& w    = s_w[cur];
 		const GemmSeg*  sg   = s_seg[cur];
 		const int       nseg = w.seg_end - w.seg_begin;
+		const int       slot = tile::warp_slot<C>(it);
 
-		if (w.kind == 0) {
-			tile::mma_tile<C>(acc, smem, a.ops, X, sg, 0, nseg, w.m0, w.n0, w.M, w.N);
+		const bool p1 = w.kind == 0;
+		if (!p1) {
+			// a pass-2 item blocks no other item: claim and fetch the next one
+			// now, behind this item's dependency wait and MMAs
 			if (warp == 0)
 				claim_next(cur ^ 1);
-			store_tile<C>(acc, a.bx + w.c_off, w.ldc, w.m0, w.n0, w.M, w.N);
+			if (tid == 0) {
+				int last_dep = -1;
+				for (int s = 0; s < nseg; ++s) {
+					const int j = sg[s].dep;
+					if (j == last_dep)
+						continue;
+					last_dep = j;
+					const unsigned target = unsigned(a.n1_of_j[j] + (j == 0 ? a.test_extra_wait : 0));
+					const unsigned long long t0 = globaltimer_ns();
+					while (ld_acquire(&a.done[j]) < target) {
+						if (ld_acquire(&a.work_counter[2]) != 0u)
+							break; // another wait already gave up
+						if (globaltimer_ns() - t0 > kWaitLimitNs) {
+							atomicExch(&a.work_counter[2], 1u);
+							*reinterpret_cast<volatile int*>(a.error) = 1;
+							__threadfence_system();
+							break;
+						}
+						__nanosleep(128);
+					}
+				}
+			}
+			__syncthreads();
+		}
+		// one inlined copy for both passes: two need 168 registers at 64 x 64
+		tile::mma_tile<C>(acc, smem, p1 ? a.ops : a.bx, p1 ? X : a.ops, sg, 0, nseg, w.m0, w.n0, w.M, w.N, it);
+		if (p1) {
+			if (warp == 0)
+				claim_next(cur ^ 1);
+			store_tile<C>(acc, a.bx + w.c_off, w.ldc, w.m0, w.n0, w.M, w.N, slot);
 			__syncthreads(); // tile stored; next descriptor visible
 			if (tid == 0) {
 				__threadfence();
@@ -150,36 +182,8 @@ __global__ void __launch_bounds__(C::THREADS) kron_persistent_kernel(PersistentA
 			}
 			continue;
 		}
-		// a pass-2 item blocks no other item: claim and fetch the next one
-		// now, behind this item's dependency wait and MMAs
-		if (warp == 0)
-			claim_next(cur ^ 1);
-		if (tid == 0) {
-			int last_dep = -1;
-			for (int s = 0; s < nseg; ++s) {
-				const int j = sg[s].dep;
-				if (j == last_dep)
-					continue;
-				last_dep = j;
-				const unsigned target = unsigned(a.n1_of_j[j] + (j == 0 ? a.test_extra_wait : 0));
-				const unsigned long long t0 = globaltimer_ns();
-				while (ld_acquire(&a.done[j]) < target) {
-					if (ld_acquire(&a.work_counter[2]) != 0u)
-						break; // another wait already gave up
-					if (globaltimer_ns() - t0 > kWaitLimitNs) {
-						atomicExch(&a.work_counter[2], 1u);
-						*reinterpret_cast<volatile int*>(a.error) = 1;
-						__threadfence_system();
-						break;
-					}
-					__nanosleep(128);
-				}
-			}
-		}
-		__syncthreads();
-		tile::mma_tile<C>(acc, smem, a.bx, a.ops, sg, 0, nseg, w.m0, w.n0, w.M, w.N);
 		if (w.kind == 1) {
-			store_tile<C>(acc, Y + w.c_off, w.ldc, w.m0, w.n0, w.M, w.N);
+			store_tile<C>(acc, Y + w.c_off, w.ldc, w.m0, w.n0, w.M, w.N, slot);
 			__syncthreads(); // next descriptor visible
 			continue;
 		}
@@ -192,7 +196,7 @@ __global__ void __launch_bounds__(C::THREADS) kron_persistent_kernel(PersistentA
 			for (int ni = 0; ni < C::NI; ++ni)
 #pragma unroll
 				for (int h = 0; h < 2; ++h)
-					part[tile::acc_col<C>(ni, h) * C::BM + tile::acc_row<C>(mi)] = acc.v[mi][ni][h];
+					part[tile::acc_col<C>(slot, ni, h) * C::BM + tile::acc_row<C>(slot, mi)] = acc.v[mi][ni][h];
 		__syncthreads();
 		if (tid == 0) {
 			__threadfence();
@@ -211,8 +215,8 @@ __global__ void __launch_bounds__(C::THREADS) kron_persistent_kernel(PersistentA
 				for (int ni = 0; ni < C::NI; ++ni)
 #pragma unroll
 					for (int h = 0; h < 2; ++h) {
-						const int r   = tile::acc_row<C>(mi);
-						const int c   = tile::acc_col<C>(ni, h);
+						const int r   = tile::acc_row<C>(slot, mi);
+						const int c   = tile::acc_col<C>(slot, ni, h);
 						const int e   = c * C::BM + r;
 						double    sum = __ldcg(slots + e);
 						for (int p = 1; p < w.nsplit; ++p)
@@ -245,7 +249,7 @@ __global__ void __launch_bounds__(C::THREADS) kron_persistent_kernel(PersistentA
 // Tile configurations a handle can run (kron_persistent.cuh, KronTileCfg).
 using PCfg0 = tile::Cfg<32, 32, 16, 16, 16, 4>;
 using PCfg1 = tile::Cfg<32, 32, 32, 16, 16, 3>;
-using PCfg2 = tile::Cfg<64, 64, 16, 32, 32, 3>;
+using PCfg2 = tile::Cfg<64, 64, 16, 32, 32, 2>;
 using PCfg3 = tile::Cfg<64, 64, 32, 32, 32, 3>;
 using PCfg4 = tile::Cfg<32, 32, 32, 16, 16, 4>;
 using PCfg5 = tile::Cfg<32, 32, 64, 16, 16, 3>;

@@ -32,7 +32,7 @@ struct PersistentArgs {
 
 // Tile configurations (output tile, k-chunk, pipeline depth):
 //   0: 32x32, k16, 4 stages   1: 32x32, k32, 3 stages
-//   2: 64x64, k16, 3 stages   3: 64x64, k32, 3 stages
+//   2: 64x64, k16, 2 stages   3: 64x64, k32, 3 stages
 //   4: 32x32, k32, 4 stages   5: 32x32, k64, 3 stages
 constexpr int kNumTileCfgs = 6;
 

@@ -327,16 +327,17 @@ void build_persistent_schedule(KronPlan& plan, int bk, int grid, int items_per_c
 	}
 	plan.n1_items = int(plan.items.size());
 
-	// K-slice length: none when the tiles alone give `items_per_cta` items per
-	// CTA, otherwise aim at that many pass-2 items per CTA, at least 4 chunks
-	// each; no item holds more than kMaxItemSegs segments
+	// K-slice length: `items_per_cta` pass-2 items per CTA on average, at
+	// least 4 chunks each; no item holds more than kMaxItemSegs segments.
+	// Sectors with more tiles than that are cut by the same rule: their few
+	// longest tiles would otherwise set the launch's end
 	long long total_k = 0;
 	for (const GemmTile& t : plan.tile2)
 		for (int s = t.seg_begin; s < t.seg_end; ++s)
 			total_k += plan.seg2[s].K;
-	long long k_target = 1LL << 40;
-	const long long want = (long long)items_per_cta * grid;
-	if ((long long)plan.tile2.size() < want && grid > 0) {
+	long long       k_target = 1LL << 40;
+	const long long want     = (long long)items_per_cta * grid;
+	if (grid > 0) {
 		k_target = total_k / want;
 		k_target = std::max<long long>(k_target, 4LL * bk);
 		k_target = (k_target + bk - 1) / bk * bk;

@@ -419,7 +419,7 @@ constexpr int kMaxItemSegs = 32;
 
 // Builds plan.items / pseg2 / n1_of_j for a persistent launch of `grid`
 // CTAs: pass-2 output tiles are cut into K-slices (multiples of bk, on any
-// k boundary) when there are fewer than items_per_cta tiles per CTA.
+// k boundary) of about the length that makes items_per_cta of them per CTA.
 void build_persistent_schedule(KronPlan& plan, int bk, int grid, int items_per_cta = 2);
 
 // Checks the persistent work list against the buffers before a launch (the
