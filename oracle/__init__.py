@@ -44,7 +44,8 @@ def build(force: bool = False) -> None:
     the reference harness."""
     if force or not os.path.exists(ORACLE_SO):
         subprocess.run(["make", "-s", "-C", HERE, "liboracle_kron.so"], check=True)
-    if os.path.isdir(REFERENCE_TREE) and (force or not os.path.exists(REF_SO)
+    if os.path.isfile(os.path.join(REFERENCE_TREE, "dmrg", "Engine", "MatrixVectorKron",
+                                   "BatchedGemmCpu.h")) and (force or not os.path.exists(REF_SO)
                                           or not os.path.exists(REF_KC_SO)):
         subprocess.run(["make", "-s", "-C", HERE, "ref", "REF=" + REFERENCE_TREE], check=True)
 
