@@ -136,6 +136,42 @@ void pick_tile(const dmrgpp_kron_desc* d, int& bm, int& bn)
 	pick_tile_sizes(d->npatches, d->left_patch_size, d->right_patch_size, bm, bn);
 }
 
+// The FP64 configuration of a new handle (the tuner replaces it by the fastest
+// on the sector itself).  Where the lines lie, from sweeps of spin links,
+// Hubbard chains and ladders and sector groups on a B200 (us per H*x):
+// * few patches, each within one fused column tile: the fused form has no
+//   dependent second pass (5 to 21 patches: 8.5 against 11.5 with two passes,
+//   12.4 against 16.5, microbench sector 27.6 against 34.8); with many small
+//   patches its units are too short (145 patches: 33 against 32), and above
+//   4e8 flops the heaviest part sets its end (6e8: 126 against 72);
+// * small work: 32 x 32 tiles with k-chunks of 32, half as many steps in the
+//   latency-bound chains (chain of 4000 states 49.3 against 56.1 with chunks
+//   of 16); from 6e8 flops shorter chunks waste less of ragged patches
+//   (batch of 8 sectors 66.5 against 70.0) unless patches are wide (ladder of
+//   10000 states, patches to 332: 445 against 460);
+// * 64 x 64 tiles only where the sector fills the SMs several times over with
+//   them: 1396 against 1449 at 3.6e10 flops, but 740 against 700 at 1.6e10
+//   and 2 to 4 times slower below 1e9.
+void default_config(const dmrgpp::KronPlan& P, int* cfg, int* ipc)
+{
+	long long widest = 0, max_l = 0;
+	for (size_t p = 0; p < P.np; ++p) {
+		max_l  = std::max(max_l, P.l[p]);
+		widest = std::max({ widest, P.l[p], P.r[p] });
+	}
+	*ipc = 2;
+	if (P.np <= 40 && max_l <= dmrgpp::fused_shape(0).bn && P.f_alg < 4e8) {
+		*cfg = dmrgpp::kNumTileCfgs;
+		*ipc = 1;
+	} else if (P.f_alg >= 2.5e10) {
+		*cfg = 2;
+	} else if (P.f_alg >= 6e8 && widest < 320) {
+		*cfg = 0;
+	} else {
+		*cfg = 1;
+	}
+}
+
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no
 // direct libcuda dependency)
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
@@ -170,9 +206,11 @@ int check_error_word(dmrgpp_kron_handle h)
 {
 	if (!h->err_host || *reinterpret_cast<volatile int*>(h->err_host) == 0)
 		return DMRGPP_OK;
-	*h->err_host      = 0;
-	const size_t nctr = 3 + h->plan.np + size_t(h->plan.n_split_tiles);
-	cudaMemsetAsync(h->d_ctr, 0, nctr * sizeof(unsigned), h->stream);
+	*h->err_host = 0;
+	if (h->d_ctr) { // a handle that only ever ran the fused form has none
+		const size_t nctr = 3 + h->plan.np + size_t(h->plan.n_split_tiles);
+		cudaMemsetAsync(h->d_ctr, 0, nctr * sizeof(unsigned), h->stream);
+	}
 	if (h->m_arrive)
 		cudaMemsetAsync(h->m_arrive, 0, size_t(std::max(h->plan.mixed.n_split_tiles, 1)) * sizeof(unsigned),
 		                h->stream);
@@ -582,7 +620,7 @@ double seconds_since(Clock::time_point t0)
 
 // t0: when create started (before the plan); the plan's time is recorded by
 // the caller in h->setup_times[DMRGPP_SETUP_PLAN]
-int finish_create(dmrgpp_kron_handle h, int device, void* stream, int bm, Clock::time_point t0,
+int finish_create(dmrgpp_kron_handle h, int device, void* stream, Clock::time_point t0,
                   dmrgpp_kron_handle* out)
 {
 	// (h->crs, when set, points at the caller's CRS operators until the upload)
@@ -622,7 +660,9 @@ int finish_create(dmrgpp_kron_handle h, int device, void* stream, int bm, Clock:
 
 	if ((e = dmrgpp::error_word_alloc(&h->err_host, &h->err_dev)))
 		return bail(e, "error word");
-	if (int rc = dmrgpp::configure_schedule(h, bm == 32 ? 0 : 2, 2)) {
+	int cfg = 0, ipc = 0;
+	default_config(P, &cfg, &ipc);
+	if (int rc = dmrgpp::configure_schedule(h, cfg, ipc)) {
 		const std::string why = h->err;
 		release(h);
 		delete h;
@@ -767,7 +807,7 @@ int dmrgpp_kron_create(const dmrgpp_kron_desc* d, dmrgpp_kron_handle* out)
 	}
 	h->sector_start                   = { 0, h->plan.dim() };
 	h->setup_times[DMRGPP_SETUP_PLAN] = seconds_since(t0);
-	return finish_create(h, d->device, d->stream, bm, t0, out);
+	return finish_create(h, d->device, d->stream, t0, out);
 }
 
 int dmrgpp_kron_create_crs(const dmrgpp_kron_crs_desc* d, dmrgpp_kron_handle* out)
@@ -806,7 +846,7 @@ int dmrgpp_kron_create_crs(const dmrgpp_kron_crs_desc* d, dmrgpp_kron_handle* ou
 	h->sector_start                   = { 0, h->plan.dim() };
 	h->setup_times[DMRGPP_SETUP_PLAN] = seconds_since(t0);
 	h->crs                            = &src; // read by finish_create's upload only
-	return finish_create(h, d->device, d->stream, bm, t0, out);
+	return finish_create(h, d->device, d->stream, t0, out);
 }
 
 int dmrgpp_kron_create_complex(const dmrgpp_kron_desc* d, dmrgpp_kron_handle* out)
@@ -982,7 +1022,7 @@ int dmrgpp_kron_create_group(const dmrgpp_kron_desc* descs, size_t nsectors, dmr
 	}
 	h->sector_start                   = std::move(starts);
 	h->setup_times[DMRGPP_SETUP_PLAN] = seconds_since(t0);
-	return finish_create(h, descs[0].device, descs[0].stream, bm, t0, out);
+	return finish_create(h, descs[0].device, descs[0].stream, t0, out);
 }
 
 int dmrgpp_kron_group_sectors(dmrgpp_kron_handle h, size_t* nsectors, long long* offsets)
@@ -1080,6 +1120,17 @@ int dmrgpp_kron_test_stall_dependency(dmrgpp_kron_handle h, int on)
 	if (!h)
 		return fail(nullptr, DMRGPP_INVALID_ARG, "null handle");
 	h->test_stall = on ? 1 : 0;
+	// the fused form has no dependency to stall: the two-pass form stands in
+	if (on && h->cfg >= dmrgpp::kNumTileCfgs) {
+		h->test_cfg = h->cfg;
+		h->test_ipc = h->items_per_cta;
+		return dmrgpp_kron_set_config(h, 0, 2);
+	}
+	if (!on && h->test_cfg >= 0) {
+		const int cfg = h->test_cfg;
+		h->test_cfg   = -1;
+		return dmrgpp_kron_set_config(h, cfg, h->test_ipc);
+	}
 	return DMRGPP_OK;
 }
 

@@ -68,6 +68,7 @@ struct dmrgpp_kron_s {
 	int*                err_host = nullptr; // mapped pinned word written by the kernel
 	int*                err_dev  = nullptr;
 	int                 test_stall = 0;     // dmrgpp_kron_test_stall_dependency
+	int                 test_cfg = -1, test_ipc = 0; // the fused configuration it replaced
 	double              setup_times[DMRGPP_SETUP_NPHASES] = {}; // dmrgpp_kron_setup_profile
 	// complex sector (dmrgpp_kron_create_complex): the plan is its real
 	// embedding with 2 np patches (real parts, then imaginary parts); user
