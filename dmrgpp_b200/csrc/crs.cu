@@ -49,9 +49,12 @@ std::string map_groups(size_t np, const size_t* off, const size_t* sz, size_t ro
 }
 
 // presence of every (i, j) block of one CRS operator (row-major np x np
-// bytes); "" or the reason the matrix is malformed
-std::string scan_crs(const dmrgpp_crs& m, size_t rows, const std::vector<int>& patch, size_t np,
-                     std::vector<unsigned char>& present)
+// bytes), and which of them are exactly the identity once scaled by value and
+// the states' parities (2: no other entry); "" or the reason the matrix is
+// malformed
+std::string scan_crs(const dmrgpp_crs& m, size_t rows, const std::vector<int>& patch, const std::vector<int>& loc,
+                     const size_t* size, size_t np, double value, const unsigned char* parity,
+                     std::vector<unsigned char>& present, std::vector<unsigned char>& ident)
 {
 	if (m.rows != rows)
 		return "operator has " + std::to_string(m.rows) + " rows, the basis " + std::to_string(rows);
@@ -60,6 +63,9 @@ std::string scan_crs(const dmrgpp_crs& m, size_t rows, const std::vector<int>& p
 	if (m.rowptr[0] != 0)
 		return "rowptr[0] must be 0";
 	present.assign(np * np, 0);
+	ident.assign(np * np, 0);
+	std::vector<int>           ones(np * np, 0);  // unit entries on the block's diagonal
+	std::vector<unsigned char> other(np * np, 0); // any other nonzero
 	std::vector<int> seen(rows, -1); // row that last used each column: repeats
 	for (size_t a = 0; a < rows; ++a) {
 		const int e0 = m.rowptr[a], e1 = m.rowptr[a + 1];
@@ -74,10 +80,22 @@ std::string scan_crs(const dmrgpp_crs& m, size_t rows, const std::vector<int>& p
 				return "column " + std::to_string(b) + " repeated in row " + std::to_string(a);
 			seen[size_t(b)] = int(a);
 			const int pj    = patch[size_t(b)];
-			if (pi >= 0 && pj >= 0 && m.values[e] != 0.0)
-				present[size_t(pi) * np + size_t(pj)] = 1;
+			if (pi >= 0 && pj >= 0 && m.values[e] != 0.0) {
+				const size_t q = size_t(pi) * np + size_t(pj);
+				present[q]     = 1;
+				const double v = m.values[e] * ((parity && parity[a]) ? -1.0 : 1.0) * value;
+				if (loc[a] == loc[size_t(b)] && v == 1.0)
+					++ones[q];
+				else if (v != 0.0)
+					other[q] = 1;
+			}
 		}
 	}
+	for (size_t i = 0; i < np; ++i)
+		for (size_t j = 0; j < np; ++j) {
+			const size_t q = i * np + j;
+			ident[q]       = size[i] == size[j] && !other[q] && size_t(ones[q]) == size[i];
+		}
 	return std::string();
 }
 
@@ -221,14 +239,15 @@ std::string crs_triples(const dmrgpp_kron_crs_desc* d, CrsSource& src, std::vect
 	if (!msg.empty())
 		return msg;
 	// presence of every block of every operator, all operators at once
-	std::vector<std::vector<unsigned char>> pa(K), pb(K);
+	std::vector<std::vector<unsigned char>> pa(K), pb(K), ia(K), ib(K);
 	std::vector<std::string>                err(2 * K);
 	parallel_for(2 * K, [&](size_t q) {
 		const size_t k = q / 2;
 		if (q % 2 == 0)
-			err[q] = scan_crs(d->A[k], nL, src.lpatch, np, pa[k]);
+			err[q] = scan_crs(d->A[k], nL, src.lpatch, src.lloc, d->left_patch_size, np, d->value ? d->value[k] : 1.0,
+			                  d->fermion && d->fermion[k] ? d->left_parity : nullptr, pa[k], ia[k]);
 		else
-			err[q] = scan_crs(d->B[k], nR, src.rpatch, np, pb[k]);
+			err[q] = scan_crs(d->B[k], nR, src.rpatch, src.rloc, d->right_patch_size, np, 1.0, nullptr, pb[k], ib[k]);
 	});
 	for (size_t q = 0; q < 2 * K; ++q)
 		if (!err[q].empty())
@@ -244,7 +263,8 @@ std::string crs_triples(const dmrgpp_kron_crs_desc* d, CrsSource& src, std::vect
 					continue;
 				lists[k * np + i].push_back({ int(j), int(triples.size()) });
 				triples.push_back({ int(i), int(j), int(k) });
-				blocks.push_back({ nullptr, 0, nullptr, 0 });
+				blocks.push_back({ nullptr, 0, nullptr, 0,
+				                   (ia[k][i * np + j] ? kIdentA : 0) | (ib[k][i * np + j] ? kIdentB : 0) });
 				f_alg += 2.0 * double(r[i]) * double(l[j]) * (double(r[j]) + double(l[i]));
 			}
 	src.tri_ptr.assign(K * np + 1, 0);

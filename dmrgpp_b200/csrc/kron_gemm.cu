@@ -13,7 +13,7 @@ __global__ void __launch_bounds__(C::THREADS) grouped_dgemm_kernel(GemmArgs args
 	extern __shared__ __align__(16) double smem[];
 	const GemmTile t = args.tiles[blockIdx.x];
 	tile::Acc<C>   acc;
-	tile::mma_tile<C>(acc, smem, args.A, args.B, args.segs, t.seg_begin, t.seg_end, t.m0, t.n0, t.M, t.N,
+	tile::mma_tile<C>(acc, smem, args.A, args.B, args.X, args.segs, t.seg_begin, t.seg_end, t.m0, t.n0, t.M, t.N,
 	                  int(blockIdx.x));
 	const int slot = tile::warp_slot<C>(int(blockIdx.x));
 	double*   Cp   = args.C + t.c_off;

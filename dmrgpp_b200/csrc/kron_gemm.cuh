@@ -24,6 +24,7 @@ struct GemmArgs {
 	const GemmSeg*  segs;
 	const GemmTile* tiles;
 	int             ntiles;
+	const double*   X = nullptr; // operand of kSegXA / kSegXB segments
 };
 
 // Raises the dynamic shared-memory limit of the kernels on the current

@@ -6,7 +6,7 @@
 // K-slice reads are complete (per-patch completion counters).  Pass-1 items
 // never wait, and an item is only dequeued after all earlier items were
 // dequeued by running CTAs, so the waits always end; they are still bounded
-// in time (kWaitLimitNs); a wait that gives up raises the abort word, which
+// in time (kWaitClocks); a wait that gives up raises the abort word, which
 // ends every other wait, and the host-visible error word, and the launch
 // runs to its end with an invalid result instead of hanging.
 //
@@ -30,16 +30,9 @@
 namespace dmrgpp {
 namespace {
 
-// Upper bound of one dependency wait (nanoseconds of %globaltimer).  A legal
+// Upper bound of one dependency wait in SM clocks (0.2 s at 2 GHz).  A legal
 // wait lasts at most one pass-1 tile (microseconds to a millisecond).
-constexpr unsigned long long kWaitLimitNs = 200ull * 1000ull * 1000ull;
-
-__device__ __forceinline__ unsigned long long globaltimer_ns()
-{
-	unsigned long long t;
-	asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-	return t;
-}
+constexpr long long kWaitClocks = 400ll * 1000ll * 1000ll;
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
 {
@@ -145,32 +138,30 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) kron_persistent_kernel(Pe
 			// now, behind this item's dependency wait and MMAs
 			if (warp == 0)
 				claim_next(cur ^ 1);
-			if (tid == 0) {
-				int last_dep = -1;
-				for (int s = 0; s < nseg; ++s) {
-					const int j = sg[s].dep;
-					if (j == last_dep)
-						continue;
-					last_dep = j;
-					const unsigned target = unsigned(a.n1_of_j[j] + (j == 0 ? a.test_extra_wait : 0));
-					const unsigned long long t0 = globaltimer_ns();
+			// one lane per segment: their counters are read in parallel, not one
+			// memory latency after the other
+			if (warp == 0 && lane < nseg) {
+				const int j = sg[lane].dep; // < 0: the operands are inputs
+				if (j >= 0) {
+					const unsigned  target = unsigned(a.n1_of_j[j] + (j == 0 ? a.test_extra_wait : 0));
+					const long long t0     = clock64();
 					while (ld_acquire(&a.done[j]) < target) {
 						if (ld_acquire(&a.work_counter[2]) != 0u)
 							break; // another wait already gave up
-						if (globaltimer_ns() - t0 > kWaitLimitNs) {
+						if (clock64() - t0 > kWaitClocks) {
 							atomicExch(&a.work_counter[2], 1u);
 							*reinterpret_cast<volatile int*>(a.error) = 1;
 							__threadfence_system();
 							break;
 						}
-						__nanosleep(128);
+						__nanosleep(32);
 					}
 				}
 			}
 			__syncthreads();
 		}
 		// one inlined copy for both passes: two need 168 registers at 64 x 64
-		tile::mma_tile<C>(acc, smem, p1 ? a.ops : a.bx, p1 ? X : a.ops, sg, 0, nseg, w.m0, w.n0, w.M, w.N, it);
+		tile::mma_tile<C>(acc, smem, p1 ? a.ops : a.bx, p1 ? X : a.ops, X, sg, 0, nseg, w.m0, w.n0, w.M, w.N, it);
 		if (p1) {
 			if (warp == 0)
 				claim_next(cur ^ 1);

@@ -37,6 +37,19 @@ bool has_nonzero(const double* m, size_t ld, size_t rows, size_t cols)
 	return false;
 }
 
+bool is_identity(const double* m, size_t ld, size_t rows, size_t cols)
+{
+	if (rows != cols)
+		return false;
+	for (size_t c = 0; c < cols; ++c) {
+		const double* col = m + c * ld;
+		for (size_t r = 0; r < rows; ++r)
+			if (col[r] != (r == c ? 1.0 : 0.0))
+				return false;
+	}
+	return true;
+}
+
 void add_tiles(std::vector<GemmTile>& tiles,
                long long              c_off,
                long long              ldc,
@@ -79,6 +92,9 @@ void order_tiles(std::vector<GemmTile>& tiles, const std::vector<GemmSeg>& segs)
 
 } // namespace
 
+// 0: B_k(i,j) X_j (A is the identity), 1: X_j A^T (B is), 2: both products
+static int term_kind(int ident) { return ident & kIdentB ? 1 : ident & kIdentA ? 0 : 2; }
+
 void build_tile_lists(KronPlan& plan, int bm, int bn)
 {
 	const size_t np = plan.np;
@@ -91,7 +107,7 @@ void build_tile_lists(KronPlan& plan, int bm, int bn)
 	plan.tile2.clear();
 	// pass 1: one segment and a tile grid per input patch with work
 	for (size_t j = 0; j < np; ++j) {
-		if (plan.M[j] == 0)
+		if (plan.M1[j] == 0)
 			continue;
 		GemmSeg s {};
 		s.a_off = plan.bstack_off[j];
@@ -102,7 +118,7 @@ void build_tile_lists(KronPlan& plan, int bm, int bn)
 		s.dep   = int(j);
 		const int sb = int(plan.seg1.size());
 		plan.seg1.push_back(s);
-		add_tiles(plan.tile1, plan.bx_off[j], plan.M[j], plan.M[j], plan.l[j], sb, sb + 1, bm, bn);
+		add_tiles(plan.tile1, plan.bx_off[j], plan.M[j], plan.M1[j], plan.l[j], sb, sb + 1, bm, bn);
 	}
 	order_tiles(plan.tile1, plan.seg1);
 
@@ -110,18 +126,43 @@ void build_tile_lists(KronPlan& plan, int bm, int bn)
 	// without contributions still gets tiles so Y_i is overwritten with 0
 	size_t t = 0;
 	for (size_t i = 0; i < np; ++i) {
-		const int sb = int(plan.seg2.size());
-		for (; t < nt && plan.triples[t].i == int(i); ++t) {
-			const Triple& tr = plan.triples[t];
-			GemmSeg       s {};
-			s.a_off = plan.bx_off[tr.j] + plan.row_off[t];
-			s.lda   = int(plan.M[tr.j]);
-			s.b_off = plan.at_off[t];
-			s.ldb   = int(plan.l[tr.j]);
-			s.K     = int(plan.l[tr.j]);
-			s.dep   = tr.j;
-			plan.seg2.push_back(s);
-		}
+		const int    sb    = int(plan.seg2.size());
+		const size_t first = t;
+		while (t < nt && plan.triples[t].i == int(i))
+			++t;
+		const size_t end = t;
+		// terms whose operands are inputs first (X as B, then X as A)
+		for (int kind = 0; kind < 3; ++kind)
+			for (size_t t = first; t < end; ++t) {
+				if (term_kind(plan.ident[t]) != kind)
+					continue;
+				const Triple& tr = plan.triples[t];
+				const int     id = plan.ident[t];
+				GemmSeg       s {};
+				if (id & kIdentB) { // Y_i += X_j A^T
+					s.a_off = plan.xy_start[tr.j];
+					s.lda   = int(plan.r[tr.j]);
+					s.b_off = plan.at_off[t];
+					s.ldb   = int(plan.l[tr.j]);
+					s.K     = int(plan.l[tr.j]);
+					s.dep   = kSegXA;
+				} else if (id & kIdentA) { // Y_i += B X_j
+					s.a_off = plan.bstack_off[tr.j] + plan.row_off[t];
+					s.lda   = int(plan.M[tr.j]);
+					s.b_off = plan.xy_start[tr.j];
+					s.ldb   = int(plan.r[tr.j]);
+					s.K     = int(plan.r[tr.j]);
+					s.dep   = kSegXB;
+				} else {
+					s.a_off = plan.bx_off[tr.j] + plan.row_off[t];
+					s.lda   = int(plan.M[tr.j]);
+					s.b_off = plan.at_off[t];
+					s.ldb   = int(plan.l[tr.j]);
+					s.K     = int(plan.l[tr.j]);
+					s.dep   = tr.j;
+				}
+				plan.seg2.push_back(s);
+			}
 		const int se = int(plan.seg2.size());
 		add_tiles(plan.tile2, plan.xy_start[i], plan.r[i], plan.r[i], plan.l[i], sb, se, bm, bn);
 	}
@@ -148,11 +189,14 @@ std::string collect_triples(size_t noperator, size_t np, const size_t* lsz, cons
 				cand.push_back(t);
 			}
 	// the all-zero test reads every block: on all host cores
-	std::vector<char> keep(cand.size(), 0);
+	std::vector<char> keep(cand.size(), 0), ident(cand.size(), 0);
 	parallel_for(cand.size(), [&](size_t q) {
 		const size_t t = cand[q];
 		const size_t i = t % np, j = (t / np) % np;
 		keep[q]        = has_nonzero(A[t], ldA[t], lsz[i], lsz[j]) && has_nonzero(B[t], ldB[t], rsz[i], rsz[j]);
+		if (keep[q])
+			ident[q] = char((is_identity(A[t], ldA[t], lsz[i], lsz[j]) ? kIdentA : 0)
+			                | (is_identity(B[t], ldB[t], rsz[i], rsz[j]) ? kIdentB : 0));
 	});
 	for (size_t q = 0; q < cand.size(); ++q) {
 		if (!keep[q])
@@ -160,7 +204,7 @@ std::string collect_triples(size_t noperator, size_t np, const size_t* lsz, cons
 		const size_t t = cand[q];
 		const size_t i = t % np, j = (t / np) % np, k = t / np2;
 		triples.push_back({ int(i) + patch_offset, int(j) + patch_offset, int(k) });
-		blocks.push_back({ A[t], ldA[t], B[t], ldB[t] });
+		blocks.push_back({ A[t], ldA[t], B[t], ldB[t], ident[q] });
 		f_alg += 2.0 * double(rsz[i]) * double(lsz[j]) * (double(rsz[j]) + double(lsz[i]));
 	}
 	return std::string();
@@ -237,17 +281,27 @@ std::string build_kron_plan_triples(size_t noperator, size_t npatches, const siz
 	}
 	plan.triples = std::move(triples);
 	plan.blocks  = std::move(blocks);
+	plan.ident.clear();
+	for (const BlockRef& b : plan.blocks)
+		plan.ident.push_back(b.ident);
 	plan.f_alg   = f_alg;
 
 	const size_t nt = plan.triples.size();
 	// pass-1 row layout: for each input patch j the rows of (i,k) stacked in
-	// (i,k) order
+	// (i,k) order, those of terms with an identity factor last
 	plan.M.assign(np, 0);
+	plan.M1.assign(np, 0);
 	plan.row_off.assign(nt, 0);
-	for (size_t t = 0; t < nt; ++t) {
-		const Triple& tr = plan.triples[t];
-		plan.row_off[t]  = plan.M[tr.j];
-		plan.M[tr.j] += plan.r[tr.i];
+	for (int ident = 0; ident < 2; ++ident) {
+		for (size_t t = 0; t < nt; ++t) {
+			if ((plan.ident[t] != 0) != (ident != 0))
+				continue;
+			const Triple& tr = plan.triples[t];
+			plan.row_off[t]  = plan.M[tr.j];
+			plan.M[tr.j] += plan.r[tr.i];
+		}
+		if (ident == 0)
+			plan.M1 = plan.M;
 	}
 	if (*std::max_element(plan.M.begin(), plan.M.end()) > INT_MAX / 2)
 		return "stacked pass-1 operator too tall";
@@ -374,8 +428,8 @@ void build_persistent_schedule(KronPlan& plan, int bk, int grid, int items_per_c
 				const GemmSeg&  g    = plan.seg2[s];
 				const long long take = std::min<long long>(need, g.K - k0);
 				GemmSeg         piece = g;
-				piece.a_off += k0 * g.lda; // A = BX_j columns k0..
-				piece.b_off += k0;         // B = A^T rows k0.. (K-contiguous)
+				piece.a_off += k0 * g.lda; // A columns k0..
+				piece.b_off += k0;         // B rows k0.. (K-contiguous)
 				piece.K = int(take);
 				plan.pseg2.push_back(piece);
 				need -= take;
@@ -465,7 +519,8 @@ std::string validate_persistent_schedule(const KronPlan& plan, int tile)
 			return at(p1 ? "BX store out of range" : "y store out of range", q);
 		for (int e = w.seg_begin; e < w.seg_end; ++e) {
 			const GemmSeg& g = segs[size_t(e)];
-			if (g.dep < 0 || size_t(g.dep) >= plan.np || g.K < 0)
+			const bool xa = !p1 && g.dep == kSegXA, xb = !p1 && g.dep == kSegXB;
+			if (g.K < 0 || (!xa && !xb && (g.dep < 0 || size_t(g.dep) >= plan.np)))
 				return at("segment dependency", q);
 			if (p1) {
 				// A: Bstack_j rows m, k < K in the operators; B: X_j k < K, columns n
@@ -474,6 +529,16 @@ std::string validate_persistent_schedule(const KronPlan& plan, int tile)
 				const long long xlo = plan.xy_start[size_t(g.dep)], xhi = plan.xy_start[size_t(g.dep) + 1];
 				if (g.K > 0 && ncols > 0 && !range_ok(g.b_off + (long long)w.n0 * g.ldb, 0, g.K, ncols, g.ldb, xlo, xhi))
 					return at("pass-1 x load out of X_j", q);
+			} else if (xa) {
+				if (!range_ok(g.a_off, w.m0, m1, g.K, g.lda, 0, dim))
+					return at("pass-2 x load out of the sector vector", q);
+				if (g.K > 0 && ncols > 0 && !range_ok(g.b_off + (long long)w.n0 * g.ldb, 0, g.K, ncols, g.ldb, 0, ops))
+					return at("pass-2 A^T load out of the operators", q);
+			} else if (xb) {
+				if (!range_ok(g.a_off, w.m0, m1, g.K, g.lda, 0, ops))
+					return at("pass-2 B load out of the operators", q);
+				if (g.K > 0 && ncols > 0 && !range_ok(g.b_off + (long long)w.n0 * g.ldb, 0, g.K, ncols, g.ldb, 0, dim))
+					return at("pass-2 x load out of the sector vector", q);
 			} else {
 				const long long blo = plan.bx_off[size_t(g.dep)];
 				const long long bhi = blo + plan.M[size_t(g.dep)] * plan.l[size_t(g.dep)];
@@ -488,7 +553,7 @@ std::string validate_persistent_schedule(const KronPlan& plan, int tile)
 			    || plan.seg1[size_t(w.seg_begin)].dep != w.producer)
 				return at("pass-1 producer", q);
 			const size_t j = size_t(w.producer);
-			if (w.c_off != plan.bx_off[j] || w.M != plan.M[j] || w.N != plan.l[j] || w.ldc != plan.M[j])
+			if (w.c_off != plan.bx_off[j] || w.M != plan.M1[j] || w.N != plan.l[j] || w.ldc != plan.M[j])
 				return at("pass-1 output is not BX_j", q);
 			area[j] += (m1 - w.m0) * ncols;
 			++n1[j];
@@ -503,7 +568,7 @@ std::string validate_persistent_schedule(const KronPlan& plan, int tile)
 		}
 	}
 	for (size_t j = 0; j < plan.np; ++j)
-		if (n1[j] != plan.n1_of_j[j] || area[j] != plan.M[j] * plan.l[j])
+		if (n1[j] != plan.n1_of_j[j] || area[j] != plan.M1[j] * plan.l[j])
 			return "pass-1 tiles do not cover BX_" + std::to_string(j) + " exactly once";
 	for (size_t s = 0; s < slot_use.size(); ++s)
 		if (slot_use[s] != 1)

@@ -11,6 +11,14 @@
 //     Y_i (r_i x l_i) = sum over (j,k) of BX_j[rows of (i,k)] * A_k(i,j)^T
 // The transposed A blocks are packed once (AT = A^T, l_j x l_i) so both
 // passes read their B operand K-contiguous.
+//
+// A term with an identity factor (H_L x I and I x H_R: two of a superblock's
+// terms in every patch) is one product, not two, and needs no pass 1: pass 2
+// takes X_j itself as its A operand where B is the identity (Y_i += X_j A^T),
+// and as its B operand where A is (Y_i += B X_j).  That is 20% of the
+// multiplications of a spin link's sector and 11 to 21% of a Hubbard ladder's
+// or chain's.  (The TF32x3
+// form multiplies the identities out.)
 #pragma once
 
 #include <algorithm>
@@ -87,8 +95,11 @@ struct alignas(16) GemmSeg {
 	int       lda;
 	int       ldb;
 	int       K;
-	int       dep; // input patch j whose pass-1 result the segment reads (pass 2)
+	int       dep; // input patch j whose pass-1 result the segment reads (pass 2), or
+	               // a kSeg* code: an operand of pass 2 is X itself, nothing to wait for
 };
+constexpr int kSegXA = -1; // A operand = X_j (B_k(i,j) is the identity), B = A^T
+constexpr int kSegXB = -2; // A operand = B_k(i,j) in Bstack_j, B = X_j (A_k(i,j) is the identity)
 
 // One CTA's output tile [m0, m0+BM) x [n0, n0+BN) of an M x N matrix at
 // c_off (leading dimension ldc), summed over segments [seg_begin, seg_end).
@@ -188,7 +199,9 @@ struct BlockRef {
 	size_t        ldA;
 	const double* B;
 	size_t        ldB;
+	int           ident = 0; // kIdentA, kIdentB: the block is exactly the identity
 };
+constexpr int kIdentA = 1, kIdentB = 2;
 
 // Layout of the mixed-precision (tensor-core) form of a sector.  Every
 // operand is a "chunked K-major" matrix: rows padded to a multiple of 8 (Rp),
@@ -240,11 +253,14 @@ struct KronPlan {
 	std::vector<long long> xy_start;    // np+1 offsets into X / Y
 	std::vector<Triple>    triples;     // contributing (i,j,k), (i,j,k) order
 	std::vector<BlockRef>  blocks;      // per triple: host blocks (create time only)
+	std::vector<int>       ident;       // per triple: kIdentA, kIdentB
 	double                 f_alg = 0.0; // sum 2 r_i l_j (r_j + l_i)
 
 	// packed operator buffer (doubles)
 	std::vector<long long> bstack_off; // per input patch j
 	std::vector<long long> M;          // rows of Bstack_j / BX_j
+	std::vector<long long> M1;         // the first of them, which pass 1 computes (the rest belong
+	                                   // to terms with an identity factor)
 	std::vector<long long> at_off;     // per triple: packed A^T block
 	long long              op_elems = 0;
 

@@ -191,7 +191,7 @@ int dmrgpp_kron_apply_noalloc(const dmrgpp_kron_desc* d, const double* x, double
 	if ((e = dmrgpp::launch_grouped_dgemm(a1, plan.bm, plan.bn, stream)))
 		return restore(noalloc_fail(DMRGPP_CUDA_ERROR,
 		                            std::string("pass 1: ") + cudaGetErrorString(e)));
-	dmrgpp::GemmArgs a2 { bx, ops, y, seg2, tile2, int(plan.tile2.size()) };
+	dmrgpp::GemmArgs a2 { bx, ops, y, seg2, tile2, int(plan.tile2.size()), x };
 	if ((e = dmrgpp::launch_grouped_dgemm(a2, plan.bm, plan.bn, stream)))
 		return restore(noalloc_fail(DMRGPP_CUDA_ERROR,
 		                            std::string("pass 2: ") + cudaGetErrorString(e)));

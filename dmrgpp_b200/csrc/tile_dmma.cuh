@@ -96,11 +96,13 @@ template <class C> __device__ __forceinline__ int warp_slot(int rot)
 // Rows and columns past the matrix are not loaded; what their shared words
 // hold only reaches outputs that are not stored.  k past the segment's end is
 // zero-filled.
+// A segment's operands lie in Abase and Bbase, or (kSegXA, kSegXB) in X.
 template <class C>
 __device__ __forceinline__ void mma_tile(Acc<C>&        acc,
                                          double*        smem,
                                          const double*  Abase,
                                          const double*  Bbase,
+                                         const double*  X,
                                          const GemmSeg* segs,
                                          int            sb,
                                          int            se,
@@ -155,8 +157,12 @@ __device__ __forceinline__ void mma_tile(Acc<C>&        acc,
 		kleft           = g.K;
 		astep           = (long long)AK * g.lda;
 		bstep           = (long long)BNS * g.ldb;
-		ap              = Abase + g.a_off + (m0 + am) + (long long)ak * g.lda;
-		bp              = Bbase + g.b_off + (long long)(n0 + bn) * g.ldb + bk;
+		// X in one operand's place; with X as B, A is the operators, which are
+		// the pass's B
+		const double* a = g.dep == kSegXA ? X : g.dep == kSegXB ? Bbase : Abase;
+		const double* b = g.dep == kSegXB ? X : Bbase;
+		ap              = a + g.a_off + (m0 + am) + (long long)ak * g.lda;
+		bp              = b + g.b_off + (long long)(n0 + bn) * g.ldb + bk;
 	};
 	auto issue = [&](int stage) {
 		while (kleft <= 0) { // an empty segment has no chunk
