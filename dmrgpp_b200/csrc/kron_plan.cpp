@@ -1211,6 +1211,10 @@ std::string build_mixed_plan(KronPlan& plan, int bn, std::vector<float>* ops_hi,
 		}
 		mp.tile2.swap(out);
 	}
+	for (GemmTile& g : mp.tile1)
+		g.chunks = int(kcost(mp.seg1, g) / 32);
+	for (GemmTile& g : mp.tile2)
+		g.chunks = int(kcost(mp.seg2, g) / 32);
 	std::stable_sort(mp.tile1.begin(), mp.tile1.end(), [&](const GemmTile& x, const GemmTile& y) {
 		return kcost(mp.seg1, x) > kcost(mp.seg1, y);
 	});

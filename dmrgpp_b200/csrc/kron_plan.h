@@ -119,6 +119,7 @@ struct alignas(16) GemmTile {
 	int       split_part;
 	int       split_tile;
 	int       slot;
+	int       chunks; // tensor-core passes: 32-wide k-chunks of the segments
 };
 
 // One work item of the persistent launch (kron_persistent.cu).

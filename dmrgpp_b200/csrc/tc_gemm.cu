@@ -17,8 +17,8 @@
 //     in the 128-byte-swizzled K-major layout tcgen05.mma reads.  The x
 //     coordinate is always 0.
 //   warp 1, one thread: MMA issuer.  Per chunk it waits for the stage's
-//     bytes, issues 3 x 4 MMAs (M = 128, N = BN, K = 8) into the tile's TMEM
-//     accumulator and commits them to the stage's "empty" mbarrier; after
+//     bytes, issues 3 x 4 MMAs (M = 128, N = the tile's columns rounded up to
+//     16, K = 8) into the tile's TMEM accumulator and commits them to the stage's "empty" mbarrier; after
 //     the tile's last chunk it commits to the accumulator's "full" mbarrier.
 //     Two accumulators (2 x BN TMEM columns) alternate between tiles, so one
 //     tile's epilogue overlaps the next tile's loads and MMAs.
@@ -72,8 +72,9 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, unsigned sr
 
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
 
-// the issuing thread's bulk stores have finished reading shared memory
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory"); }
+// all but the issuing thread's last bulk store have finished reading shared
+// memory
+__device__ __forceinline__ void bulk_wait_read_1() { asm volatile("cp.async.bulk.wait_group.read 1;\n" ::: "memory"); }
 
 // the issuing thread's bulk stores are complete (written to global memory)
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
@@ -88,9 +89,10 @@ __device__ __forceinline__ void st_shared_v4(unsigned addr, float a, float b, fl
 }
 
 // instruction descriptor, kind::tf32: D = F32, A = B = TF32, both K-major
-template <int BN> __device__ __forceinline__ unsigned idesc_tf32()
+// n columns (a multiple of 16)
+__device__ __forceinline__ unsigned idesc_tf32(int n)
 {
-	return (1u << 4) | (2u << 7) | (2u << 10) | (unsigned(BN >> 3) << 17) | (unsigned(kBM >> 4) << 24);
+	return (1u << 4) | (2u << 7) | (2u << 10) | (unsigned(n >> 3) << 17) | (unsigned(kBM >> 4) << 24);
 }
 
 __device__ __forceinline__ void mma_tf32(unsigned d, uint64_t a, uint64_t b, unsigned idesc, unsigned acc)
@@ -114,14 +116,6 @@ template <int BN> struct TcLayout {
 	static constexpr int B_BYTES     = BN * 128;
 	static constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
 };
-
-__device__ __forceinline__ int tile_chunks(const TcArgs& a, const GemmTile& t)
-{
-	int n = 0;
-	for (int s = t.seg_begin; s < t.seg_end; ++s)
-		n += a.segs[s].K / kBK;
-	return n;
-}
 
 __device__ __forceinline__ void give_up(volatile int* abort, int* error)
 {
@@ -147,12 +141,30 @@ __device__ void producer(const TcArgs& a, unsigned base, unsigned full0, unsigne
 	bool     ok = true;
 	// a tiled load moves its whole box (rows past the buffer arrive as 0)
 	constexpr unsigned kStageTx = 2u * unsigned(L::A_BYTES + L::B_BYTES);
-	for (int ti = a.starts[blockIdx.x]; ti < a.starts[blockIdx.x + 1] && ok; ++ti) {
-		if (skip_tile(a, ti))
-			continue;
-		const GemmTile t = a.tiles[ti];
+	const int          end      = a.starts[blockIdx.x + 1];
+	auto               active   = [&](int ti) { // the first tile from ti on that is not skipped
+		while (ti < end && skip_tile(a, ti))
+			++ti;
+		return ti;
+	};
+	// tiles and segments are read one ahead, behind the waits and copies of the
+	// current one
+	int      ti = active(a.starts[blockIdx.x]);
+	GemmTile tn {};
+	if (ti < end)
+		tn = a.tiles[ti];
+	while (ti < end && ok) {
+		const GemmTile t = tn;
+		ti               = active(ti + 1);
+		if (ti < end)
+			tn = a.tiles[ti];
+		GemmSeg next {};
+		if (t.seg_begin < t.seg_end)
+			next = a.segs[t.seg_begin];
 		for (int s = t.seg_begin; s < t.seg_end && ok; ++s) {
-			const GemmSeg sg   = a.segs[s];
+			const GemmSeg sg = next;
+			if (s + 1 < t.seg_end)
+				next = a.segs[s + 1];
 			const int     nk   = sg.K / kBK;
 			const int     arow = int(sg.a_off) + t.m0; // buffer row of chunk 0
 			const int     brow = int(sg.b_off) + t.n0;
@@ -196,7 +208,6 @@ __device__ void mma_issuer(const TcArgs& a, unsigned base, unsigned tmem, unsign
                            volatile int* abort)
 {
 	using L               = TcLayout<BN>;
-	const unsigned idesc  = idesc_tf32<BN>();
 	unsigned       g      = 0; // chunks consumed
 	unsigned       tc     = 0; // tiles accumulated
 	bool           ok     = true;
@@ -205,10 +216,12 @@ __device__ void mma_issuer(const TcArgs& a, unsigned base, unsigned tmem, unsign
 		if (skip_tile(a, ti))
 			continue;
 		const GemmTile t     = a.tiles[ti];
-		const int      total = tile_chunks(a, t);
+		const int      total = t.chunks;
 		if (total == 0)
 			continue;
-		const unsigned b = tc & 1;
+		// only the columns that exist: a ragged tile's MMAs end sooner
+		const unsigned idesc = idesc_tf32((min(BN, t.N - t.n0) + 15) & ~15);
+		const unsigned b     = tc & 1;
 		if (tc >= 2 && !mbar_wait(acce0 + 8 * b, ((tc >> 1) - 1) & 1, abort)) {
 			ok = false;
 			break;
@@ -302,30 +315,32 @@ __device__ __forceinline__ void store_chunk_tma(const TcArgs& a, const GemmTile&
 	const int col0 = t.n0 + c0;
 	if (col0 >= t.N)
 		return;
-	if (lane == 0)
-		bulk_wait_read(); // the previous chunk's stores have read the tile
-	__syncwarp();
+	// hi and lo in tiles of their own: each is refilled while the other's store
+	// is on its way
 	const unsigned rowaddr = stg + unsigned(lane) * 128u;
+	const int      R       = int(t.c_off >> 5) + (col0 >> 5) * t.ldc + t.m0 + row0;
 #pragma unroll
-	for (int q = 0; q < 8; ++q) {
-		float hv[4], lv[4];
+	for (int part = 0; part < 2; ++part) {
+		if (lane == 0)
+			bulk_wait_read_1(); // this tile's previous store has read it
+		__syncwarp();
 #pragma unroll
-		for (int e = 0; e < 4; ++e) {
-			const float x = (col0 + 4 * q + e < t.N) ? v[4 * q + e] : 0.f;
-			hv[e]         = tf32_rna(x);
-			lv[e]         = tf32_rna(x - hv[e]);
+		for (int q = 0; q < 8; ++q) {
+			float o[4];
+#pragma unroll
+			for (int e = 0; e < 4; ++e) {
+				const float x = (col0 + 4 * q + e < t.N) ? v[4 * q + e] : 0.f;
+				const float h = tf32_rna(x);
+				o[e]          = part == 0 ? h : tf32_rna(x - h);
+			}
+			st_shared_v4(rowaddr + unsigned(part) * 4096u + unsigned((q ^ (lane & 7)) << 4), o[0], o[1], o[2], o[3]);
 		}
-		const unsigned off = unsigned((q ^ (lane & 7)) << 4);
-		st_shared_v4(rowaddr + off, hv[0], hv[1], hv[2], hv[3]);
-		st_shared_v4(rowaddr + 4096u + off, lv[0], lv[1], lv[2], lv[3]);
-	}
-	fence_proxy_async();
-	__syncwarp();
-	if (lane == 0) {
-		const int R = int(t.c_off >> 5) + (col0 >> 5) * t.ldc + t.m0 + row0;
-		tma_store_2d(&a.C_hi_map, stg, R);
-		tma_store_2d(&a.C_lo_map, stg + 4096u, R);
-		bulk_commit();
+		fence_proxy_async();
+		__syncwarp();
+		if (lane == 0) {
+			tma_store_2d(part == 0 ? &a.C_hi_map : &a.C_lo_map, stg + unsigned(part) * 4096u, R);
+			bulk_commit();
+		}
 	}
 }
 
@@ -348,49 +363,46 @@ __device__ __forceinline__ bool epilogue_all(bool v)
 }
 
 // part of a K-split pass-2 tile: this thread's row of one 32-column chunk
-// into the part's FP32 slot (row-major 128 x BN)
+// into the part's FP32 slot (column-major 128 x BN: a warp's rows are
+// adjacent, one 128-byte line per column; only what the matrix has)
 template <int BN>
-__device__ __forceinline__ void store_partial(const TcArgs& a, const GemmTile& t, int row, int c0,
+__device__ __forceinline__ void store_partial(const TcArgs& a, const GemmTile& t, int row, int c0, int vn,
                                               const float (&v)[32])
 {
-	float* dst = a.partial + (size_t(t.slot + t.split_part) * 128 + size_t(row)) * BN + c0;
+	if (t.m0 + row >= t.M)
+		return;
+	float* dst = a.partial + (size_t(t.slot + t.split_part) * BN + size_t(c0)) * 128 + size_t(row);
 #pragma unroll
-	for (int q = 0; q < 8; ++q)
-		reinterpret_cast<float4*>(dst)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+	for (int i = 0; i < 32; ++i)
+		if (c0 + i < vn)
+			dst[i * 128] = v[i];
 }
 
 // after every part of split tile t wrote its slot: sum the slots in part
 // order (deterministic) and write y
 template <int BN>
-__device__ __forceinline__ void reduce_split(const TcArgs& a, const GemmTile& t, int row)
+__device__ __forceinline__ void reduce_split(const TcArgs& a, const GemmTile& t, int row, int vn)
 {
 	const int grow = t.m0 + row;
 	if (grow >= t.M)
 		return;
 	double* y = (a.io ? a.io->y : a.Cd) + t.c_off;
-	for (int c0 = 0; c0 < BN && t.n0 + c0 < t.N; c0 += 32) {
+	for (int c0 = 0; c0 < vn; c0 += 32) {
 		float s[32];
 #pragma unroll
 		for (int i = 0; i < 32; ++i)
 			s[i] = 0.f;
 		for (int p = 0; p < t.nsplit; ++p) {
-			const float4* src = reinterpret_cast<const float4*>(
-			    a.partial + (size_t(t.slot + p) * 128 + size_t(row)) * BN + c0);
+			const float* src = a.partial + (size_t(t.slot + p) * BN + size_t(c0)) * 128 + size_t(row);
 #pragma unroll
-			for (int q = 0; q < 8; ++q) {
-				const float4 f = __ldcg(src + q);
-				s[4 * q] += f.x;
-				s[4 * q + 1] += f.y;
-				s[4 * q + 2] += f.z;
-				s[4 * q + 3] += f.w;
-			}
+			for (int i = 0; i < 32; ++i)
+				if (c0 + i < vn)
+					s[i] += __ldcg(src + i * 128);
 		}
 #pragma unroll
-		for (int i = 0; i < 32; ++i) {
-			const int gcol = t.n0 + c0 + i;
-			if (gcol < t.N)
-				y[(long long)gcol * t.ldc + grow] = double(s[i]);
-		}
+		for (int i = 0; i < 32; ++i)
+			if (c0 + i < vn)
+				y[(long long)(t.n0 + c0 + i) * t.ldc + grow] = double(s[i]);
 	}
 }
 
@@ -409,7 +421,8 @@ __device__ void epilogue(const TcArgs& a, unsigned tmem, unsigned accf0, unsigne
 		if (skip_tile(a, ti))
 			continue;
 		const GemmTile t     = a.tiles[ti];
-		const int      total = tile_chunks(a, t);
+		const int      total = t.chunks;
+		const int      vn    = min(BN, t.N - t.n0); // columns inside the matrix
 		const int      grow  = t.m0 + row;
 		float          v[32];
 		if (total == 0) { // output tile without terms: zeros
@@ -432,10 +445,10 @@ __device__ void epilogue(const TcArgs& a, unsigned tmem, unsigned accf0, unsigne
 		// pass 1: this warp's 32 rows all inside the matrix (the same for
 		// every lane) -> staged TMA stores; a partial row group stores directly
 		const bool staged = PASS1 && t.m0 + quarter * 32 + 32 <= t.M;
-		for (int c0 = 0; c0 < BN; c0 += 32) {
+		for (int c0 = 0; c0 < vn; c0 += 32) {
 			tmem_ld32(tmem + (unsigned(quarter * 32) << 16) + b * unsigned(BN) + unsigned(c0), v);
 			if (split)
-				store_partial<BN>(a, t, row, c0, v);
+				store_partial<BN>(a, t, row, c0, vn, v);
 			else if (staged)
 				store_chunk_tma<BN>(a, t, quarter * 32, c0, v, stg, lane);
 			else
@@ -458,7 +471,7 @@ __device__ void epilogue(const TcArgs& a, unsigned tmem, unsigned accf0, unsigne
 			}
 			epilogue_sync();
 			if (s_last) {
-				reduce_split<BN>(a, t, row);
+				reduce_split<BN>(a, t, row, vn);
 				epilogue_sync();
 				if (threadIdx.x == 64)
 					a.arrive[t.split_tile] = 0u; // ready for the next launch
