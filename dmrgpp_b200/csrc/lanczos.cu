@@ -40,6 +40,7 @@ constexpr int kThreads   = 256;
 constexpr int kMaxBlocks = 1184; // 8 per SM of a B200
 constexpr int kDotGrid   = 592;  // blocks of the basis projections (4 per SM)
 constexpr int kDotChunk  = 2048; // rows per block iteration of the basis projections
+constexpr int kShortChunk = 512; // and of sectors with fewer such chunks than blocks
 constexpr int kMaxCols   = 1024; // stored Lanczos vectors per solve
 
 // blocks of the row-parallel basis kernels: at least 256 rows each
@@ -185,12 +186,52 @@ __global__ void __launch_bounds__(kThreads) k_scale_inv(double* v, size_t n, con
 	scale_inv_body(v, n, s);
 }
 
+// acc[c] += <V[0..len), c], vs[0..len)> for c < ncols, one chunk of at most
+// CHUNK rows staged in shared memory: every warp streams whole columns (warp w:
+// columns w, w + 8, ...).  VEC: 16-byte loads (V, v 16-byte aligned and ld
+// even), 4 to 8 loads in flight per lane.  The order of every sum is fixed, so
+// results are bitwise reproducible.
+template <bool VEC, int CHUNK>
+__device__ __forceinline__ void project_chunk(const double* __restrict__ V, size_t ld, int ncols,
+                                              const double* vs, int len, double* acc, int lane, int warp)
+{
+	for (int c = warp; c < ncols; c += kThreads / 32) {
+		const double* col = V + size_t(c) * ld;
+		double        s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+		if (VEC && len == CHUNK) {
+			const double2* c2 = reinterpret_cast<const double2*>(col);
+			const double2* v2 = reinterpret_cast<const double2*>(vs);
+#pragma unroll 2
+			for (int q = lane; q < CHUNK / 2; q += 128) {
+				const double2 a0 = __ldg(c2 + q), a1 = __ldg(c2 + q + 32);
+				const double2 a2 = __ldg(c2 + q + 64), a3 = __ldg(c2 + q + 96);
+				const double2 b0 = v2[q], b1 = v2[q + 32], b2 = v2[q + 64], b3 = v2[q + 96];
+				s0 += a0.x * b0.x + a0.y * b0.y;
+				s1 += a1.x * b1.x + a1.y * b1.y;
+				s2 += a2.x * b2.x + a2.y * b2.y;
+				s3 += a3.x * b3.x + a3.y * b3.y;
+			}
+		} else {
+			int i = lane;
+			for (; i + 96 < len; i += 128) {
+				s0 += col[i] * vs[i];
+				s1 += col[i + 32] * vs[i + 32];
+				s2 += col[i + 64] * vs[i + 64];
+				s3 += col[i + 96] * vs[i + 96];
+			}
+			for (; i < len; i += 32)
+				s0 += col[i] * vs[i];
+		}
+		double s = (s0 + s1) + (s2 + s3);
+		for (int o = 16; o > 0; o >>= 1)
+			s += __shfl_down_sync(0xffffffffu, s, o);
+		if (lane == 0)
+			acc[c] += s;
+	}
+}
+
 // Per-block partial projections partial[b][c] = <V[rows of b, c], v[rows of b]>
-// for c < ncols.  Block b takes the kDotChunk-row chunks b, b + grid, ...;
-// each chunk of v is staged in shared memory and every warp streams whole
-// columns of it (warp w: columns w, w + 8, ...).  VEC: 16-byte loads (V, v
-// 16-byte aligned and ld even), 8 loads in flight per lane.  The order of
-// every sum is fixed, so results are bitwise reproducible.
+// for c < ncols.  Block b takes the kDotChunk-row chunks b, b + grid, ...
 template <bool VEC>
 __device__ __forceinline__ void basis_dots_body(const double* __restrict__ V, size_t ld, int ncols,
                                                 const double* __restrict__ v, size_t n,
@@ -207,39 +248,7 @@ __device__ __forceinline__ void basis_dots_body(const double* __restrict__ V, si
 		for (int i = threadIdx.x; i < len; i += kThreads)
 			vs[i] = v[base + i];
 		__syncthreads();
-		for (int c = warp; c < ncols; c += kThreads / 32) {
-			const double* col = V + size_t(c) * ld + base;
-			double        s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-			if (VEC && len == kDotChunk) {
-				const double2* c2 = reinterpret_cast<const double2*>(col);
-				const double2* v2 = reinterpret_cast<const double2*>(vs);
-#pragma unroll 2
-				for (int q = lane; q < kDotChunk / 2; q += 128) {
-					const double2 a0 = __ldg(c2 + q), a1 = __ldg(c2 + q + 32);
-					const double2 a2 = __ldg(c2 + q + 64), a3 = __ldg(c2 + q + 96);
-					const double2 b0 = v2[q], b1 = v2[q + 32], b2 = v2[q + 64], b3 = v2[q + 96];
-					s0 += a0.x * b0.x + a0.y * b0.y;
-					s1 += a1.x * b1.x + a1.y * b1.y;
-					s2 += a2.x * b2.x + a2.y * b2.y;
-					s3 += a3.x * b3.x + a3.y * b3.y;
-				}
-			} else {
-				int i = lane;
-				for (; i + 96 < len; i += 128) {
-					s0 += col[i] * vs[i];
-					s1 += col[i + 32] * vs[i + 32];
-					s2 += col[i + 64] * vs[i + 64];
-					s3 += col[i + 96] * vs[i + 96];
-				}
-				for (; i < len; i += 32)
-					s0 += col[i] * vs[i];
-			}
-			double s = (s0 + s1) + (s2 + s3);
-			for (int o = 16; o > 0; o >>= 1)
-				s += __shfl_down_sync(0xffffffffu, s, o);
-			if (lane == 0)
-				acc[c] += s;
-		}
+		project_chunk<VEC, kDotChunk>(V + base, ld, ncols, vs, len, acc, lane, warp);
 	}
 	__syncthreads();
 	for (int c = threadIdx.x; c < ncols; c += kThreads)
@@ -254,10 +263,10 @@ k_basis_dots(const double* __restrict__ V, size_t ld, int ncols, const double* _
 	basis_dots_body<VEC>(V, ld, ncols, v, n, partial);
 }
 
-// r[c] = sum over blocks b < nblocks of partial[b][c], one block per column,
+// r[c] = f * sum over blocks b < nblocks of partial[b][c], one block per column,
 // fixed order
 __device__ __forceinline__ void reduce_cols_body(const double* __restrict__ partial, int nblocks,
-                                                 double* __restrict__ r)
+                                                 double* __restrict__ r, double f = 1.0)
 {
 	__shared__ double red[kThreads / 32];
 	const int         c = blockIdx.x;
@@ -266,7 +275,7 @@ __device__ __forceinline__ void reduce_cols_body(const double* __restrict__ part
 		s += partial[size_t(b) * kMaxCols + c];
 	s = block_sum(s, red);
 	if (threadIdx.x == 0)
-		r[c] = s;
+		r[c] = f * s;
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -275,14 +284,14 @@ k_reduce_cols(const double* __restrict__ partial, int nblocks, double* __restric
 	reduce_cols_body(partial, nblocks, r);
 }
 
-// v -= V[:, 0..ncols) r ; *nrm_out = |v|.  VEC: each thread owns row pairs
+// v = f v - V[:, 0..ncols) r ; *nrm_out = |v|.  VEC: each thread owns row pairs
 // (16-byte loads), 8 columns of loads issued before their updates; the
 // subtractions run in column order, as in the scalar form.
 template <bool VEC>
 __device__ __forceinline__ void basis_subtract_body(double* __restrict__ v, const double* __restrict__ V,
                                                     size_t ld, int ncols, const double* __restrict__ r,
                                                     size_t n, double* nrm_out, double* partial,
-                                                    unsigned* ctr)
+                                                    unsigned* ctr, double f = 1.0)
 {
 	__shared__ double rs[kMaxCols];
 	__shared__ double red[kThreads / 32];
@@ -297,7 +306,9 @@ __device__ __forceinline__ void basis_subtract_body(double* __restrict__ v, cons
 		const size_t np2 = n / 2;
 		for (size_t p = first; p < np2; p += stride) {
 			double2 w = v2[p];
-			int     c = 0;
+			w.x *= f;
+			w.y *= f;
+			int c = 0;
 			for (; c + 8 <= ncols; c += 8) {
 				double2 a[8];
 #pragma unroll
@@ -319,7 +330,7 @@ __device__ __forceinline__ void basis_subtract_body(double* __restrict__ v, cons
 		}
 		if ((n & 1) && first == 0) { // odd length: the last element
 			const size_t i = n - 1;
-			double       w = v[i];
+			double       w = f * v[i];
 			for (int c = 0; c < ncols; ++c)
 				w -= V[size_t(c) * ld + i] * rs[c];
 			v[i] = w;
@@ -327,7 +338,7 @@ __device__ __forceinline__ void basis_subtract_body(double* __restrict__ v, cons
 		}
 	} else {
 		for (size_t i = first; i < n; i += stride) {
-			double w = v[i];
+			double w = f * v[i];
 			for (int c = 0; c < ncols; ++c)
 				w -= V[size_t(c) * ld + i] * rs[c];
 			v[i] = w;
@@ -349,8 +360,16 @@ k_basis_subtract(double* __restrict__ v, const double* __restrict__ V, size_t ld
 
 // ---- one Lanczos step with its columns chosen on the device, so that a
 // captured CUDA graph of check_every steps is replayed unchanged for the
-// whole solve.  k_step_advance moves the step record to the next j before
-// every step (LanczosVectors::oneStepDecomposition, LanczosVectors.h:203-241).
+// whole solve.  The last kernel of a step moves the step record to the next j
+// (LanczosVectors::oneStepDecomposition, LanczosVectors.h:203-241).
+//
+// Small sectors are bound by the launches' latencies and by how many SMs each
+// pass fills, so a step is five kernels after the H*x: alpha; the update with
+// |v2| and the projections of its result in one pass (the chunk of v2 is in
+// shared memory anyway); the columns' sums; the subtraction, which also
+// applies the first 1/beta; the second scaling.  Eight kernels and projections
+// on one block per 2048 rows took 39 us a step at 98,000 rows and 30 columns,
+// five with one block per 512 rows 27 us.
 struct LanczosStep {
 	StepIO  io;      // the step's H*x: x = V_j, y = V_{j+1}
 	double* v0;      // V_{j-1}
@@ -363,11 +382,8 @@ struct LanczosStep {
 	int     j;
 };
 
-__global__ void k_step_set(LanczosStep* sp, int j) { sp->j = j; }
-
-__global__ void k_step_advance(LanczosStep* sp, double* V, size_t D, double* alpha, double* beta)
+__device__ __forceinline__ void step_to(LanczosStep* sp, int j, double* V, size_t D, double* alpha, double* beta)
 {
-	const int j = sp->j + 1;
 	sp->j       = j;
 	sp->v0      = V + size_t(j - 1) * D;
 	sp->v1      = V + size_t(j) * D;
@@ -378,6 +394,11 @@ __global__ void k_step_advance(LanczosStep* sp, double* V, size_t D, double* alp
 	sp->beta_j  = beta + j;
 	sp->beta_j1 = beta + j + 1;
 	sp->ncols   = j + 1;
+}
+
+__global__ void k_step_set(LanczosStep* sp, int j, double* V, size_t D, double* alpha, double* beta)
+{
+	step_to(sp, j, V, D, alpha, beta);
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -392,29 +413,69 @@ k_update_step(const LanczosStep* sp, size_t n, double* partial, unsigned* ctr)
 	update_body(sp->v2, sp->v1, sp->v0, n, sp->alpha_j, sp->beta_j, sp->beta_j1, partial, ctr);
 }
 
-// v2 *= 1 / *s (s = beta_{j+1} when null)
+// 1 / s, or 1 when s is not positive (LanczosVectors.h:233-237)
+__device__ __forceinline__ double inv_or_one(double s) { return s > 0.0 ? 1.0 / s : 1.0; }
+
+// v2 *= 1 / *s (s = beta_{j+1} when null), and the step record moves on once
+// every block has read it
 __global__ void __launch_bounds__(kThreads)
-k_scale_inv_step(const LanczosStep* sp, size_t n, const double* s)
+k_scale_advance_step(LanczosStep* sp, size_t n, const double* s, double* V, double* alpha, double* beta,
+                     unsigned* ctr)
 {
+	const int j = sp->j;
 	scale_inv_body(sp->v2, n, s ? s : sp->beta_j1);
+	__syncthreads();
+	if (threadIdx.x == 0 && last_block(ctr))
+		step_to(sp, j + 1, V, n, alpha, beta);
 }
 
-template <bool VEC>
+// The update v2 -= alpha v1 + beta v0, *beta_{j+1} = |v2|, and the block's
+// partial projections partial[b][c] = <V[rows of b, c], v2[rows of b]>,
+// c < ncols, in one pass: block b takes the CHUNK-row chunks b, b + grid, ...
+template <bool VEC, int CHUNK>
 __global__ void __launch_bounds__(kThreads, 4)
-k_basis_dots_step(const LanczosStep* sp, const double* __restrict__ V, size_t ld, size_t n,
-                  double* __restrict__ partial)
+k_update_dots_step(const LanczosStep* sp, const double* __restrict__ V, size_t ld, size_t n,
+                   double* __restrict__ partial, double* norm_partial, unsigned* ctr)
 {
-	basis_dots_body<VEC>(V, ld, sp->ncols, sp->v2, n, partial);
+	__shared__ __align__(16) double vs[CHUNK];
+	__shared__ double               acc[kMaxCols];
+	__shared__ double               red[kThreads / 32];
+	double* __restrict__ v2       = sp->v2;
+	const double* __restrict__ v1 = sp->v1;
+	const double* __restrict__ v0 = sp->v0;
+	const double a = *sp->alpha_j, b = *sp->beta_j;
+	const int    ncols = sp->ncols, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	double       nrm = 0.0;
+	for (int c = threadIdx.x; c < ncols; c += kThreads)
+		acc[c] = 0.0;
+	for (size_t base = size_t(blockIdx.x) * CHUNK; base < n; base += size_t(gridDim.x) * CHUNK) {
+		const int len = int(std::min<size_t>(CHUNK, n - base));
+		__syncthreads();
+		for (int i = threadIdx.x; i < len; i += kThreads) {
+			const double w = v2[base + i] - a * v1[base + i] - b * v0[base + i];
+			v2[base + i]   = w;
+			vs[i]          = w;
+			nrm += w * w;
+		}
+		__syncthreads();
+		project_chunk<VEC, CHUNK>(V + base, ld, ncols, vs, len, acc, lane, warp);
+	}
+	__syncthreads();
+	for (int c = threadIdx.x; c < ncols; c += kThreads)
+		partial[size_t(blockIdx.x) * kMaxCols + c] = acc[c];
+	nrm = block_sum(nrm, red);
+	grid_sum(nrm, norm_partial, ctr, sp->beta_j1, true, red);
 }
 
-// launched with the largest column count; blocks past the step's ncols exit
+// r[c] = <V_c, v2> / beta_{j+1}; launched with the largest column count, blocks
+// past the step's ncols exit
 __global__ void __launch_bounds__(kThreads)
 k_reduce_cols_step(const LanczosStep* sp, const double* __restrict__ partial, int nblocks,
                    double* __restrict__ r)
 {
 	if (int(blockIdx.x) >= sp->ncols)
 		return;
-	reduce_cols_body(partial, nblocks, r);
+	reduce_cols_body(partial, nblocks, r, inv_or_one(*sp->beta_j1));
 }
 
 template <bool VEC>
@@ -423,7 +484,7 @@ k_basis_subtract_step(const LanczosStep* sp, const double* __restrict__ V, size_
                       const double* __restrict__ r, size_t n, double* nrm_out, double* partial,
                       unsigned* ctr)
 {
-	basis_subtract_body<VEC>(sp->v2, V, ld, sp->ncols, r, n, nrm_out, partial, ctr);
+	basis_subtract_body<VEC>(sp->v2, V, ld, sp->ncols, r, n, nrm_out, partial, ctr, inv_or_one(*sp->beta_j1));
 }
 
 // z = sum_c coef[c] V[:, c] (LanczosVectors::excitedVector, LanczosVectors.h:192-201)
@@ -736,38 +797,39 @@ int dmrgpp_lanczos_lowest(dmrgpp_kron_handle          h,
 	                                          w->partial, w->ctr + 2);
 	k_scale_inv<<<nb, kThreads, 0, st>>>(col(1), D, beta + 1);
 
-	// graph-replayed steps: every kernel of a step reads its columns from the
-	// step record, so one captured graph of check_every steps serves the
-	// whole solve (same kernels and grids as the launches below: bitwise
-	// identical results)
+	// every kernel of a step reads its columns from the step record, so one
+	// captured graph of check_every steps serves the whole solve (the same
+	// kernels and grids launch by launch: bitwise identical results)
 	LanczosStep* sp       = static_cast<LanczosStep*>(w->step);
 	const bool   vec      = vec2_ok(V, V + D, D);
-	const int    dgrid    = int(std::max<size_t>(1, std::min<size_t>((D + kDotChunk - 1) / kDotChunk, kDotGrid)));
-	const int    sgrid    = basis_blocks_for(D);
-	const bool   use_graph = p->use_graph != 0;
+	// short chunks until there are blocks enough to fill the SMs
+	const bool   short_chunks = D < size_t(kDotChunk) * kDotGrid;
+	const size_t chunk        = short_chunks ? kShortChunk : kDotChunk;
+	const int    dgrid        = int(std::max<size_t>(1, std::min<size_t>((D + chunk - 1) / chunk, kDotGrid)));
+	const int    sgrid        = basis_blocks_for(D);
+	const bool   use_graph    = p->use_graph != 0;
+	double*      norms        = w->partial + size_t(kDotGrid) * kMaxCols; // behind the columns' partials
 	auto         enqueue_step = [&](cudaStream_t s) -> int {
-		k_step_advance<<<1, 1, 0, s>>>(sp, V, D, alpha, beta);
 		if (int rc = kron_apply_device(h, nullptr, nullptr, &sp->io))
 			return rc;
 		k_dot_step<<<nb, kThreads, 0, s>>>(sp, D, w->partial, w->ctr + 1);
-		k_update_step<<<nb, kThreads, 0, s>>>(sp, D, w->partial, w->ctr + 2);
-		k_scale_inv_step<<<nb, kThreads, 0, s>>>(sp, D, nullptr);
-		if (p->reortho) {
-			if (vec) {
-				k_basis_dots_step<true><<<dgrid, kThreads, 0, s>>>(sp, V, D, D, w->partial);
-			} else {
-				k_basis_dots_step<false><<<dgrid, kThreads, 0, s>>>(sp, V, D, D, w->partial);
-			}
-			k_reduce_cols_step<<<w->cols, kThreads, 0, s>>>(sp, w->partial, dgrid, w->r);
-			if (vec) {
-				k_basis_subtract_step<true><<<sgrid, kThreads, 0, s>>>(sp, V, D, w->r, D, work + 1,
-				                                                      w->partial, w->ctr + 4);
-			} else {
-				k_basis_subtract_step<false><<<sgrid, kThreads, 0, s>>>(sp, V, D, w->r, D, work + 1,
-				                                                       w->partial, w->ctr + 4);
-			}
-			k_scale_inv_step<<<nb, kThreads, 0, s>>>(sp, D, work + 1);
+		if (!p->reortho) {
+			k_update_step<<<nb, kThreads, 0, s>>>(sp, D, w->partial, w->ctr + 2);
+			k_scale_advance_step<<<nb, kThreads, 0, s>>>(sp, D, nullptr, V, alpha, beta, w->ctr + 5);
+			return DMRGPP_OK;
 		}
+		auto dots = vec ? (short_chunks ? k_update_dots_step<true, kShortChunk> : k_update_dots_step<true, kDotChunk>)
+		                : (short_chunks ? k_update_dots_step<false, kShortChunk> : k_update_dots_step<false, kDotChunk>);
+		dots<<<dgrid, kThreads, 0, s>>>(sp, V, D, D, w->partial, norms, w->ctr + 2);
+		k_reduce_cols_step<<<w->cols, kThreads, 0, s>>>(sp, w->partial, dgrid, w->r);
+		if (vec) {
+			k_basis_subtract_step<true><<<sgrid, kThreads, 0, s>>>(sp, V, D, w->r, D, work + 1, w->partial,
+			                                                      w->ctr + 4);
+		} else {
+			k_basis_subtract_step<false><<<sgrid, kThreads, 0, s>>>(sp, V, D, w->r, D, work + 1, w->partial,
+			                                                       w->ctr + 4);
+		}
+		k_scale_advance_step<<<nb, kThreads, 0, s>>>(sp, D, work + 1, V, alpha, beta, w->ctr + 5);
 		return DMRGPP_OK;
 	};
 	struct Graph {
@@ -806,46 +868,24 @@ int dmrgpp_lanczos_lowest(dmrgpp_kron_handle          h,
 			rc = cuda_status(h, e, "graph instantiation");
 		return rc;
 	};
-	if (use_graph)
-		k_step_set<<<1, 1, 0, st>>>(sp, 0); // the first step is j = 1
+	k_step_set<<<1, 1, 0, st>>>(sp, 1, V, D, alpha, beta);
 
 	// Groups of check_every steps are enqueued one group ahead of the host's
 	// stopping test (two pinned copies of alpha/beta alternate), so the GPU
 	// runs the next group while the host tests the last one; steps past the
 	// stopping point are discarded, as in the one-group-at-a-time form.
 	auto enqueue_group = [&](size_t j0, size_t j1) -> int {
-		if (use_graph) {
-			if (j1 - j0 == size_t(p->check_every)) {
-				if (!graph.x)
-					if (int rc = capture())
-						return rc;
-				if ((e = cudaGraphLaunch(graph.x, st)))
-					return cuda_status(h, e, "graph launch");
-			} else {
-				for (size_t jj = j0; jj < j1; ++jj)
-					if (int rc = enqueue_step(st))
-						return rc;
-			}
+		if (use_graph && j1 - j0 == size_t(p->check_every)) {
+			if (!graph.x)
+				if (int rc = capture())
+					return rc;
+			if ((e = cudaGraphLaunch(graph.x, st)))
+				return cuda_status(h, e, "graph launch");
 			return DMRGPP_OK;
 		}
-		for (size_t jj = j0; jj < j1; ++jj) {
-			// oneStepDecomposition (LanczosVectors.h:203-241), V2 lives in column jj+1
-			double* v0 = col(jj - 1);
-			double* v1 = col(jj);
-			double* v2 = col(jj + 1);
-			if (int rc = kron_apply_device(h, v1, v2))
+		for (size_t jj = j0; jj < j1; ++jj)
+			if (int rc = enqueue_step(st))
 				return rc;
-			k_dot<<<nb, kThreads, 0, st>>>(v2, v1, D, alpha + jj, w->partial, w->ctr + 1);
-			k_lanczos_update<<<nb, kThreads, 0, st>>>(v2, v1, v0, D, alpha + jj, beta + jj,
-			                                          beta + jj + 1, w->partial, w->ctr + 2);
-			k_scale_inv<<<nb, kThreads, 0, st>>>(v2, D, beta + jj + 1);
-			if (p->reortho) { // reorthoIfNecessary (LanczosVectors.h:243-271)
-				const int nc = int(jj) + 1;
-				basis_dots(V, D, nc, v2, D, w->r, w->partial, st);
-				basis_subtract(v2, V, D, nc, w->r, D, work + 1, w->partial, w->ctr + 4, st);
-				k_scale_inv<<<nb, kThreads, 0, st>>>(v2, D, work + 1);
-			}
-		}
 		return DMRGPP_OK;
 	};
 	struct Events {
