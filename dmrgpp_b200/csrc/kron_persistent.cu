@@ -240,8 +240,8 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) kron_persistent_kernel(Pe
 // Tile configurations a handle can run (kron_persistent.cuh, KronTileCfg).
 using PCfg0 = tile::Cfg<32, 32, 16, 16, 16, 4>;
 using PCfg1 = tile::Cfg<32, 32, 32, 16, 16, 3>;
-using PCfg2 = tile::Cfg<64, 64, 16, 32, 32, 2>;
-using PCfg3 = tile::Cfg<64, 64, 32, 32, 32, 3>;
+using PCfg2 = tile::Cfg<64, 64, 16, 32, 32, 2, true>;
+using PCfg3 = tile::Cfg<64, 64, 32, 32, 32, 3, true>;
 using PCfg4 = tile::Cfg<32, 32, 32, 16, 16, 4>;
 using PCfg5 = tile::Cfg<32, 32, 64, 16, 16, 3>;
 

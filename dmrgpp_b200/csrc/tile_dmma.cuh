@@ -25,6 +25,18 @@ __device__ __forceinline__ void cp_async_8(unsigned dst, const double* src, bool
 	             : "memory");
 }
 
+// The same where `issue` holds; nothing at all otherwise (the predicate is
+// inside: a branch around each copy costs more than the copy).
+__device__ __forceinline__ void cp_async_8_if(bool issue, unsigned dst, const double* src, bool pred)
+{
+	const int n = pred ? 8 : 0;
+	asm volatile("{\n\t.reg .pred p;\n\t"
+	             "setp.ne.b32 p, %3, 0;\n\t"
+	             "@p cp.async.ca.shared.global [%0], [%1], 8, %2;\n\t}\n" ::"r"(dst),
+	             "l"(src), "r"(n), "r"(int(issue))
+	             : "memory");
+}
+
 __device__ __forceinline__ void cp_async_commit()
 {
 	asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -44,8 +56,14 @@ __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, dou
 	             : "d"(a), "d"(b));
 }
 
-template <int BM_, int BN_, int BK_, int WM_, int WN_, int STAGES_> struct Cfg {
+// SKIP: rows and columns past the matrix are not copied at all.  Otherwise the
+// copy engine zero-fills them, which takes fewer predicates: better where
+// latency counts (ladder of 6000 states with 32 x 32 tiles 139 us against 148,
+// transformation of 4000 states 35 against 37), worse for the persistent 64 x
+// 64 tiles, whose registers are full (16000 states 1347 against 1309).
+template <int BM_, int BN_, int BK_, int WM_, int WN_, int STAGES_, bool SKIP_ = false> struct Cfg {
 	static constexpr int BM = BM_, BN = BN_, BK = BK_, WM = WM_, WN = WN_, STAGES = STAGES_;
+	static constexpr bool SKIP = SKIP_;
 	static constexpr int WARPS_M = BM / WM, WARPS_N = BN / WN;
 	static constexpr int THREADS = WARPS_M * WARPS_N * 32;
 	static constexpr int MI = WM / 8, NI = WN / 8;
@@ -93,9 +111,9 @@ template <class C> __device__ __forceinline__ int warp_slot(int rot)
 // * `rot` turns the warps' places in the tile: a ragged tile leaves the same
 //   places empty, and each scheduler's share of the pipe has to see all of
 //   them in turn.
-// Rows and columns past the matrix are not loaded; what their shared words
-// hold only reaches outputs that are not stored.  k past the segment's end is
-// zero-filled.
+// Rows and columns past the matrix are zero-filled or (Cfg's SKIP) not loaded;
+// what their shared words hold only reaches outputs that are not stored.  k
+// past the segment's end is zero-filled.
 // A segment's operands lie in Abase and Bbase, or (kSegXA, kSegXB) in X.
 template <class C>
 __device__ __forceinline__ void mma_tile(Acc<C>&        acc,
@@ -175,8 +193,10 @@ __device__ __forceinline__ void mma_tile(Acc<C>&        acc,
 #pragma unroll
 		for (int e = 0; e < C::A_LOADS; ++e) {
 			const bool in = ak + e * AK < kleft;
-			if (arow)
-				cp_async_8(da + unsigned(e * AK * C::LDA_S * 8), in ? p : Abase, in);
+			if (C::SKIP)
+				cp_async_8_if(arow, da + unsigned(e * AK * C::LDA_S * 8), in ? p : Abase, in);
+			else
+				cp_async_8(da + unsigned(e * AK * C::LDA_S * 8), in && arow ? p : Abase, in && arow);
 			p += astep;
 		}
 		ap                = p;
@@ -184,8 +204,11 @@ __device__ __forceinline__ void mma_tile(Acc<C>&        acc,
 		const bool    kin = bk < kleft;
 #pragma unroll
 		for (int e = 0; e < C::B_LOADS; ++e) {
-			if (e * BNS < ncol)
-				cp_async_8(db + unsigned(e * BNS * C::LDB_S * 8), kin ? q : Bbase, kin);
+			const bool cin = e * BNS < ncol;
+			if (C::SKIP)
+				cp_async_8_if(cin, db + unsigned(e * BNS * C::LDB_S * 8), kin ? q : Bbase, kin);
+			else
+				cp_async_8(db + unsigned(e * BNS * C::LDB_S * 8), kin && cin ? q : Bbase, kin && cin);
 			q += bstep;
 		}
 		bp += C::BK;
@@ -232,9 +255,14 @@ __device__ __forceinline__ void mma_tile(Acc<C>&        acc,
 						dmma_8x8x4(acc.v[mi][ni][0], acc.v[mi][ni][1], af[mi], bf[ni]);
 			}
 		} else if (vm > 0 && vn > 0) {
+			// unrolled: the next step's fragment loads overlap this one's MMAs
+			// (one at a time, a transformation of patches below a tile took 18
+			// us instead of 14)
 			const int kv = min(ck, C::BK);
-#pragma unroll 1
-			for (int ks = 0; ks < kv; ks += 4) {
+#pragma unroll
+			for (int ks = 0; ks < C::BK; ks += 4) {
+				if (ks >= kv)
+					break;
 				double af[C::MI], bf[C::NI];
 #pragma unroll
 				for (int mi = 0; mi < C::MI; ++mi)

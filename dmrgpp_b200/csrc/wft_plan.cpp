@@ -76,7 +76,12 @@ std::string build_wft_plan(const dmrgpp_wft_desc& d, WftPlan& plan, std::vector<
 	}
 	if (plan.x_start.back() > (long long)INT_MAX * 64 || plan.y_start.back() > (long long)INT_MAX * 64)
 		return "sector too large";
-	plan.bm = plan.bn = maxs > 192 ? 64 : 32;
+	// 64 x 64 tiles where they fill the SMs with four CTAs each; smaller layouts
+	// are latency-bound and want more, smaller tiles
+	long long tiles64 = 0;
+	for (size_t q = 0; q < d.np_out; ++q)
+		tiles64 += ((plan.l_out[q] + 63) / 64) * ((plan.r_out[q] + 63) / 64);
+	plan.bm = plan.bn = maxs > 192 && tiles64 >= 4 * 148 ? 64 : 32;
 
 	// packed blocks and the intermediate T
 	plan.wr_off.assign(d.np_out, 0);
