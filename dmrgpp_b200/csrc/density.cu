@@ -9,11 +9,11 @@
 // density-matrix eigenvalues are the squared singular values and the kept
 // transformation is U.  Here rho_g = M_g M_g^T is formed directly as a sum of
 // X_p^T X_p (system side) or X_p X_p^T (environment side) by one grouped DGEMM
-// launch on the FP64 tensor pipe, the rho_g come to the host, are reduced to
-// tridiagonal form and their eigenvalues found there, group by group on the
-// host cores (Householder and implicit QL, tridiag.cpp), the eigenvectors are
-// formed on the device from the recorded QL rotations and Householder
-// reflectors, and the kept number follows computeKeptStates.
+// launch on the FP64 tensor pipe and reduced to tridiagonal form there, one
+// cluster of CTAs per group, their eigenvalues found by bisection; the host
+// ranks the states (computeKeptStates) and forms the kept eigenvectors of the
+// tridiagonals by inverse iteration on all cores (tridiag.cpp), and the device
+// applies the Householder reflectors to them.
 #include "devmem.h"
 #include "trace.h"
 #include "dmrgpp_kron.h"
@@ -21,6 +21,7 @@
 #include "kron_gemm.cuh"
 #include "tridiag.h"
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -65,11 +66,357 @@ k_transpose_tiles(const double* __restrict__ x, double* __restrict__ xt, const T
 	}
 }
 
-// Eigenvectors on the device.  The host reduces each rho_g to tridiagonal
-// form (Householder reflectors h_k, beta_k), finds all its eigenvalues (QL
-// without vectors), ranks the states, and for the kept ones only computes
-// the tridiagonal eigenvectors Z by inverse iteration; the device applies the
-// reflectors to them (V = Q Z), the O(n^2) per vector part of the work.
+namespace cg = cooperative_groups;
+
+// One group of the tridiagonal reduction.
+struct TridiagJob {
+	long long m_off; // rho_g (n x n)
+	long long e_off; // its place in the per-state arrays
+	int       n;
+	int       group;
+};
+
+constexpr int kTriCluster = 8;
+constexpr int kTriThreads = 512;
+constexpr int kTriMaxN    = 2048; // largest group (its vectors are in shared memory)
+
+// sum over the block, the same in every thread (fixed order)
+__device__ __forceinline__ double block_sum_all(double v, double* red)
+{
+	for (int o = 16; o > 0; o >>= 1)
+		v += __shfl_xor_sync(0xffffffffu, v, o);
+	__syncthreads(); // red free
+	if ((threadIdx.x & 31) == 0)
+		red[threadIdx.x >> 5] = v;
+	__syncthreads();
+	double s = 0.0;
+#pragma unroll
+	for (int w = 0; w < kTriThreads / 32; ++w)
+		s += red[w];
+	return s;
+}
+
+// Householder reduction of rho_g to tridiagonal form, T = Q^T rho Q with
+// householder_tridiag's conventions (tridiag.cpp): diagonal d, off-diagonal
+// off, reflectors h_k into column k of rho_g's own storage, beta.  One cluster
+// of 8 CTAs per group; CTA r owns columns r, r + 8, ... of the working copy
+// `work` (both triangles).  A step makes one pass over the owned trailing
+// columns that applies the previous step's rank-2 update and forms this step's
+// product y = A h (one warp per column, so y needs no sum across CTAs), sends
+// y to all CTAs' shared memory and meets them at one cluster barrier; the
+// column that makes the next reflector, its norm, and the vectors h and q are
+// formed by every CTA for itself.  All groups run side by side: the launch
+// lasts as long as the largest group's n steps of a few memory latencies each
+// (the host cores took 10.6 ms for 241 groups of up to 532 states with their
+// eigenvalues, this kernel 3.8).
+__global__ void __cluster_dims__(kTriCluster, 1, 1) __launch_bounds__(kTriThreads)
+k_tridiag(double* __restrict__ rho, double* __restrict__ work, const TridiagJob* __restrict__ jobs, double* d,
+          double* off, double* beta, int* shift, int vec)
+{
+	extern __shared__ __align__(16) double smem[];
+	__shared__ double                      red[kTriThreads / 32];
+	__shared__ double                      amax_of[kTriCluster];
+	cg::cluster_group                      cluster = cg::this_cluster();
+	const int                              rank    = int(cluster.block_rank());
+	const int                              tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	const TridiagJob                       jb = jobs[blockIdx.x / kTriCluster];
+	const int                              n  = jb.n;
+	double*                                R  = rho + jb.m_off;
+	double*                                A  = work + jb.m_off;
+	d += jb.e_off;
+	off += jb.e_off;
+	beta += jb.e_off;
+	// vectors of the step, `vec` doubles each: column and new h, previous h
+	// and q (index 0 = row k), and y of this and the previous step
+	double* h  = smem;
+	double* hp = smem + vec;
+	double* qp = smem + 2 * vec;
+	double* y2 = smem + 3 * vec;
+
+	// working copy, symmetrised; the largest entry outside [2^-64, 2^64]:
+	// 2^shift rho instead (group_eigenvalues has the reason)
+	double amax = 0.0;
+	for (int c = rank + kTriCluster * warp; c < n; c += kTriCluster * (kTriThreads / 32))
+		for (int i = lane; i < n; i += 32) {
+			const double v = 0.5 * (R[i + (long long)c * n] + R[c + (long long)i * n]);
+			A[i + (long long)c * n] = v;
+			amax                    = fmax(amax, fabs(v));
+		}
+	for (int o = 16; o > 0; o >>= 1)
+		amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+	if (lane == 0)
+		red[warp] = amax;
+	__syncthreads();
+	if (tid < kTriCluster) {
+		double m = 0.0;
+		for (int w = 0; w < kTriThreads / 32; ++w)
+			m = fmax(m, red[w]);
+		*cluster.map_shared_rank(&amax_of[rank], tid) = m;
+	}
+	cluster.sync(); // every copy of rho_g is read, every maximum is here
+	amax = 0.0;
+	for (int r = 0; r < kTriCluster; ++r)
+		amax = fmax(amax, amax_of[r]);
+	int sh = 0;
+	if (amax > 0.0 && isfinite(amax) && (amax < 0x1p-64 || amax > 0x1p64)) {
+		int e = 0;
+		frexp(amax, &e);
+		sh = -e;
+		for (int c = rank + kTriCluster * warp; c < n; c += kTriCluster * (kTriThreads / 32))
+			for (int i = lane; i < n; i += 32)
+				A[i + (long long)c * n] = ldexp(A[i + (long long)c * n], sh);
+		cluster.sync();
+	}
+	if (rank == 0 && tid == 0)
+		shift[jb.group] = sh;
+
+	bool pending = false; // A <- A - hp qp^T - qp hp^T on rows / columns >= k
+	for (int k = 0; k + 2 < n; ++k) {
+		const int len = n - k - 1;
+		double*   y   = y2 + (k & 1) * vec;
+		// column k, rows k .. n-1, brought up to date (its owner wrote it in an
+		// earlier step: read from L2)
+		const double hk = pending ? hp[0] : 0.0, qk = pending ? qp[0] : 0.0;
+		double       sigma = 0.0, dk = 0.0;
+		for (int i = tid; i <= len; i += kTriThreads) {
+			double v = __ldcg(A + (k + i) + (long long)k * n);
+			if (pending)
+				v -= hp[i] * qk + qp[i] * hk;
+			if (i == 0)
+				dk = v;
+			else
+				h[i - 1] = v;
+			if (i >= 2)
+				sigma += v * v;
+		}
+		sigma           = block_sum_all(sigma, red); // and h is complete
+		const double x0 = h[0];
+		double       b = 0.0, h0 = 0.0, offk = x0;
+		if (sigma != 0.0) {
+			const double mu = sqrt(x0 * x0 + sigma);
+			h0              = x0 <= 0.0 ? x0 - mu : -sigma / (x0 + mu);
+			b               = 2.0 * h0 * h0 / (sigma + h0 * h0);
+			offk            = mu;
+		}
+		__syncthreads(); // x0 read by all before h changes
+		if (b != 0.0)
+			for (int i = tid; i < len; i += kTriThreads)
+				h[i] = i == 0 ? 1.0 : h[i] / h0;
+		if (rank == 0) {
+			if (tid == 0) {
+				d[k]    = dk;
+				off[k]  = offk;
+				beta[k] = b;
+			}
+			if (b != 0.0) // rho_g itself is no longer needed
+				for (int i = tid; i < len; i += kTriThreads)
+					R[i + (long long)k * n] = h[i]; // each thread its own entries
+		}
+		__syncthreads();
+		// the pass over the owned columns c > k
+		const int first = k + 1 + ((rank - (k + 1)) & (kTriCluster - 1)); // first column with c % 8 == rank
+		if (pending || b != 0.0)
+			// two columns at a time, eight loads of a lane in flight: a column is
+			// a few memory latencies long, and there are 8 x 16 of them at once
+			for (int c = first + 2 * kTriCluster * warp; c < n; c += 2 * kTriCluster * (kTriThreads / 32)) {
+				const int    c1  = c + kTriCluster;
+				const bool   two = c1 < n;
+				double*      a0  = A + (k + 1) + (long long)c * n;
+				double*      a1  = two ? A + (k + 1) + (long long)c1 * n : a0;
+				const double h0j = pending ? hp[c - k] : 0.0, q0j = pending ? qp[c - k] : 0.0;
+				const double h1j = pending && two ? hp[c1 - k] : 0.0, q1j = pending && two ? qp[c1 - k] : 0.0;
+				double       s0 = 0.0, s1 = 0.0;
+				for (int i0 = lane; i0 < len; i0 += 128) {
+					double v0[4], v1[4];
+#pragma unroll
+					for (int u = 0; u < 4; ++u) {
+						const int i = i0 + 32 * u;
+						v0[u]       = i < len ? a0[i] : 0.0;
+						v1[u]       = i < len ? a1[i] : 0.0;
+					}
+#pragma unroll
+					for (int u = 0; u < 4; ++u) {
+						const int i = i0 + 32 * u;
+						if (i < len) {
+							if (pending) {
+								const double hi = hp[i + 1], qi = qp[i + 1];
+								v0[u] -= hi * q0j + qi * h0j;
+								v1[u] -= hi * q1j + qi * h1j;
+								a0[i] = v0[u];
+								if (two)
+									a1[i] = v1[u];
+							}
+							s0 += v0[u] * h[i];
+							s1 += v1[u] * h[i];
+						}
+					}
+				}
+				for (int o = 16; o > 0; o >>= 1) {
+					s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+					s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+				}
+				if (lane < kTriCluster) {
+					double* yr    = cluster.map_shared_rank(y, lane);
+					yr[c - k - 1] = s0;
+					if (two)
+						yr[c1 - k - 1] = s1;
+				}
+			}
+		cluster.sync();
+		pending = b != 0.0;
+		if (!pending)
+			continue; // (uniform over the cluster)
+		double ph = 0.0;
+		for (int i = tid; i < len; i += kTriThreads) {
+			const double p = b * y[i];
+			y[i]           = p;
+			ph += p * h[i];
+		}
+		ph = block_sum_all(ph, red);
+		for (int i = tid; i < len; i += kTriThreads) {
+			const double hi = h[i];
+			qp[i]           = y[i] - 0.5 * b * ph * hi;
+			hp[i]           = hi;
+		}
+		__syncthreads();
+	}
+	if (rank == 0 && tid == 0) {
+		if (n == 1) {
+			d[0]    = A[0];
+			off[0]  = 0.0;
+			beta[0] = 0.0;
+		} else {
+			const int k0 = n - 2;
+			double    a00 = __ldcg(A + k0 + (long long)k0 * n), a10 = __ldcg(A + k0 + 1 + (long long)k0 * n),
+			       a11 = __ldcg(A + k0 + 1 + (long long)(k0 + 1) * n);
+			if (pending) {
+				a00 -= 2.0 * hp[0] * qp[0];
+				a10 -= hp[1] * qp[0] + qp[1] * hp[0];
+				a11 -= 2.0 * hp[1] * qp[1];
+			}
+			d[n - 2]    = a00;
+			d[n - 1]    = a11;
+			off[n - 2]  = a10;
+			off[n - 1]  = 0.0;
+			beta[n - 2] = beta[n - 1] = 0.0;
+		}
+	}
+	cluster.sync(); // no CTA leaves while another may still write to its shared memory
+}
+
+// Eigenvalues of the tridiagonals, ascending, by Sturm counts: 8 lanes count
+// at 8 points of an eigenvalue's interval at once, until the interval is below
+// 2^-55 of the norm or an ulp.  n dependent steps a count set the time, so
+// fewer rounds beat fewer counts, and the counts are sign changes of the
+// leading minors p_i+1 = (d_i - x) p_i - off_i-1^2 p_i-1 (two dependent
+// multiply-adds a step; the pivots' quotients, sturm_count in tridiag.cpp, take
+// a division: 0.66 against 1.02 ms for 16000 eigenvalues of groups up to 532).
+// The matrix is scaled to a norm of about 1, so a step multiplies the minors by
+// at most 3, and every 8 steps both are scaled back by a power of two.
+struct BisectJob {
+	long long e_off;
+	int       n, k0; // eigenvalues k0 .. k0 + 31 of the group
+};
+
+constexpr int kBisThreads = 256;
+
+__global__ void __launch_bounds__(kBisThreads)
+k_bisect(const double* __restrict__ d, const double* __restrict__ off, double* __restrict__ w,
+         const BisectJob* __restrict__ jobs)
+{
+	extern __shared__ __align__(16) double smem[];
+	__shared__ double                      lo_s[kBisThreads / 32], hi_s[kBisThreads / 32], sc_s[kBisThreads / 32];
+	const BisectJob jb = jobs[blockIdx.x];
+	const int       n = jb.n, tid = threadIdx.x, lane = tid & 31;
+	double*         ds = smem;
+	double*         e2 = smem + n; // off[i]^2
+	double          lo = 1.7e308, hi = -1.7e308, sc = 0.0;
+	for (int i = tid; i < n; i += kBisThreads) {
+		const double di = d[jb.e_off + i], oi = i + 1 < n ? off[jb.e_off + i] : 0.0;
+		const double om = i > 0 ? off[jb.e_off + i - 1] : 0.0;
+		const double r  = fabs(om) + fabs(oi);
+		ds[i]           = di;
+		e2[i]           = oi * oi;
+		lo              = fmin(lo, di - r);
+		hi              = fmax(hi, di + r);
+		sc              = fmax(sc, fabs(di) + r);
+	}
+	for (int o = 16; o > 0; o >>= 1) {
+		lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+		hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+		sc = fmax(sc, __shfl_xor_sync(0xffffffffu, sc, o));
+	}
+	if (lane == 0) {
+		lo_s[tid >> 5] = lo;
+		hi_s[tid >> 5] = hi;
+		sc_s[tid >> 5] = sc;
+	}
+	__syncthreads();
+	for (int q = 0; q < kBisThreads / 32; ++q) {
+		lo = fmin(lo, lo_s[q]);
+		hi = fmax(hi, hi_s[q]);
+		sc = fmax(sc, sc_s[q]);
+	}
+	const int k = jb.k0 + (tid >> 3); // this lane group's eigenvalue
+	if (jb.k0 >= n)
+		return;
+	const int    kk   = min(k, n - 1) + 1; // idle groups repeat the last
+	if (!(sc > 0.0)) { // the zero matrix, or not a number: lo says which
+		if ((lane & 7) == 0 && k < n)
+			w[jb.e_off + k] = lo;
+		return; // (the whole block)
+	}
+	// 2^-e T, exactly
+	int e = 0;
+	frexp(sc, &e);
+	__syncthreads();
+	for (int i = tid; i < n; i += kBisThreads) {
+		ds[i] = ldexp(ds[i], -e);
+		e2[i] = ldexp(e2[i], -2 * e);
+	}
+	__syncthreads();
+	sc = ldexp(sc, -e);
+	lo = ldexp(lo, -e) - 1e-14 * sc;
+	hi = ldexp(hi, -e) + 1e-14 * sc;
+	const int sub = lane & 7;
+	for (int it = 0; it < 200; ++it) {
+		const double gap = hi - lo;
+		if (!__any_sync(0xffffffffu, gap > 0x1p-55 * sc && lo + 0.5 * gap > lo && lo + 0.5 * gap < hi))
+			break;
+		const double x = lo + gap * (double(sub + 1) / 9.0);
+		int          c = 0;
+		double       p0 = 0.0, p1 = 1.0, f = 0.0; // p_{i-1}, p_i, off_{i-1}^2
+		for (int i0 = 0; i0 < n; i0 += 8) {
+			const int i1 = min(i0 + 8, n);
+			for (int i = i0; i < i1; ++i) {
+				double p2 = (ds[i] - x) * p1 - f * p0;
+				if (p2 == 0.0) // a zero minor has the sign opposite to its predecessor's
+					p2 = p1 < 0.0 ? 1e-280 : -1e-280;
+				c += (p2 < 0.0) != (p1 < 0.0);
+				f  = e2[i];
+				p0 = p1;
+				p1 = p2;
+			}
+			// the larger one back to [1, 2)
+			const int ex = ilogb(fmax(fabs(p0), fabs(p1)));
+			p0           = ldexp(p0, -ex);
+			p1           = ldexp(p1, -ex);
+		}
+		// the first point with kk or more eigenvalues below it bounds it above
+		const unsigned m  = (__ballot_sync(0xffffffffu, c >= kk) >> (lane & 24)) & 0xffu;
+		const int      at = m ? __ffs(m) - 1 : 8;
+		const double   xl = __shfl_sync(0xffffffffu, x, (lane & 24) + max(at - 1, 0));
+		const double   xh = __shfl_sync(0xffffffffu, x, (lane & 24) + min(at, 7));
+		lo                = at > 0 ? xl : lo;
+		hi                = at < 8 ? xh : hi;
+	}
+	if (sub == 0 && k < n)
+		w[jb.e_off + k] = ldexp(0.5 * (lo + hi), e);
+}
+
+// Eigenvectors.  For the kept states only, the host computes the tridiagonal
+// eigenvectors Z by inverse iteration; the device applies the reflectors to
+// them (V = Q Z), the O(n^2) per vector part of the work.
 
 // V[:, j] = Q Z[:, j] for every kept column j of every group: one warp per
 // column, the reflectors h_k (k = n-3 .. 0) applied in turn to the column in
@@ -352,37 +699,125 @@ extern "C" int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, d
 		if ((e = launch_grouped_dgemm(ga, bm, bm, st)))
 			return cuda_fail(e, "density-matrix GEMM launch");
 	}
-	double* h_rho = pinned<double>(0, rho_elems);
-	if (!h_rho)
-		return fail(DMRGPP_OOM, "page-locked host buffer for the density matrices");
-	if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(h_rho, rho, rho_elems * sizeof(double), cudaMemcpyDeviceToHost, st))
-	    || (e = cudaStreamSynchronize(st)))
-		return cuda_fail(e, "density matrices");
-
-	g_trunc_times[DMRGPP_TRUNC_RHO] = seconds_since(t_start);
-	auto tp                         = Clock::now();
-	// eigenvalues of every group on the host cores (Householder reduction,
-	// QL without vectors)
 	std::vector<long long> eoff(ng + 1, 0);
 	for (size_t g = 0; g < ng; ++g)
 		eoff[g + 1] = eoff[g] + (long long)d->group_size[g];
-	// largest groups first (the order of the eigenvector work below)
+	// largest groups first
 	std::vector<size_t> by_size(ng);
 	std::iota(by_size.begin(), by_size.end(), size_t(0));
 	std::stable_sort(by_size.begin(), by_size.end(),
 	                 [&](size_t x, size_t y) { return d->group_size[x] > d->group_size[y]; });
-	std::vector<double*> ga(ng), gw(ng);
-	for (size_t g = 0; g < ng; ++g) {
-		ga[g] = h_rho + goff[g];
-		gw[g] = eigenvalues + eoff[g];
-	}
 	std::vector<GroupReduction> ge;
 	const int                   hw = host_threads();
-	if (!group_eigenvalues(ng, d->group_size, ga.data(), gw.data(), ge, hw)) {
-		size_t g = 0;
-		while (g < ng && ge[g].ok)
-			++g;
-		return fail(DMRGPP_NOT_CONVERGED, "eigensolver of group " + std::to_string(g) + " did not converge");
+	auto                        not_converged = [&](size_t g) {
+        return fail(DMRGPP_NOT_CONVERGED, "eigensolver of group " + std::to_string(g) + " did not converge");
+	};
+	// reduction and eigenvalues on the device; groups whose vectors do not fit
+	// its shared memory make the host cores do it
+	const bool  on_device = nmax <= size_t(kTriMaxN);
+	double *    work = nullptr, *tri = nullptr; // tri: d, off, eigenvalues, beta (N each)
+	void*       d_tj = nullptr;
+	struct FreeT {
+		double **a, **b;
+		void**   c;
+		~FreeT()
+		{
+			dev_free(*a);
+			dev_free(*b);
+			dev_free(*c);
+		}
+	} freet { &work, &tri, &d_tj };
+	Clock::time_point tp;
+	if (on_device) {
+		if ((e = cudaGetLastError()))
+			return cuda_fail(e, "density matrices");
+		std::vector<TridiagJob> tj;
+		std::vector<BisectJob>  bj;
+		for (size_t g : by_size) {
+			const int n = int(d->group_size[g]);
+			if (n == 0)
+				continue;
+			tj.push_back({ goff[g], eoff[g], n, int(g) });
+			for (int k0 = 0; k0 < n; k0 += kBisThreads / 8)
+				bj.push_back({ eoff[g], n, k0 });
+		}
+		// the lists and the groups' shifts in one allocation
+		const size_t tjb = tj.size() * sizeof(TridiagJob), bjb = bj.size() * sizeof(BisectJob);
+		std::vector<unsigned char> lists(tjb + bjb);
+		std::copy_n(reinterpret_cast<const unsigned char*>(tj.data()), tjb, lists.data());
+		std::copy_n(reinterpret_cast<const unsigned char*>(bj.data()), bjb, lists.data() + tjb);
+		const size_t N1 = std::max<size_t>(N, 1);
+		double*      h_tri = pinned<double>(0, 3 * N1 + (ng + 1) / 2 + 1);
+		if (!h_tri)
+			return fail(DMRGPP_OOM, "page-locked host buffer for the tridiagonals");
+		int*       h_shift = reinterpret_cast<int*>(h_tri + 3 * N1);
+		const int  vec     = int(std::max<size_t>(nmax, 1));
+		const size_t tri_smem = 5 * size_t(vec) * sizeof(double), bis_smem = 2 * size_t(vec) * sizeof(double);
+		if ((e = dev_malloc(&work, rho_elems * sizeof(double))) || (e = dev_malloc(&tri, 4 * N1 * sizeof(double)))
+		    || (e = dev_malloc(&d_tj, lists.size() + ng * sizeof(int) + 16))
+		    || (e = cudaFuncSetAttribute(k_tridiag, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		                                 int(5 * size_t(kTriMaxN) * sizeof(double)))))
+			return cuda_fail(e, "tridiagonal allocation");
+		unsigned char* lp      = static_cast<unsigned char*>(d_tj);
+		int*           d_shift = reinterpret_cast<int*>(lp + lists.size());
+		if (!lists.empty() && (e = cudaMemcpyAsync(lp, lists.data(), lists.size(), cudaMemcpyHostToDevice, st)))
+			return cuda_fail(e, "tridiagonal set-up");
+		double *dd = tri, *doff = tri + N1, *dw = tri + 2 * N1, *dbeta = tri + 3 * N1;
+		if (!tj.empty()) {
+			k_tridiag<<<unsigned(tj.size() * kTriCluster), kTriThreads, tri_smem, st>>>(
+			    rho, work, reinterpret_cast<const TridiagJob*>(lp), dd, doff, dbeta, d_shift, vec);
+			k_bisect<<<unsigned(bj.size()), kBisThreads, bis_smem, st>>>(
+			    dd, doff, dw, reinterpret_cast<const BisectJob*>(lp + tjb));
+		}
+		if ((e = cudaGetLastError())
+		    || (e = cudaMemcpyAsync(h_tri, tri, 3 * N1 * sizeof(double), cudaMemcpyDeviceToHost, st))
+		    || (e = cudaMemcpyAsync(h_shift, d_shift, ng * sizeof(int), cudaMemcpyDeviceToHost, st)))
+			return cuda_fail(e, "tridiagonal reduction");
+		g_trunc_times[DMRGPP_TRUNC_RHO] = seconds_since(t_start);
+		tp                              = Clock::now();
+		if ((e = cudaStreamSynchronize(st)))
+			return cuda_fail(e, "tridiagonal reduction");
+		ge.assign(ng, GroupReduction {});
+		for (size_t g = 0; g < ng; ++g) {
+			const size_t n = d->group_size[g];
+			if (n == 0)
+				continue;
+			GroupReduction& r = ge[g];
+			const double *  gd = h_tri + eoff[g], *go = gd + N1, *gv = go + N1;
+			r.d.assign(gd, gd + n);
+			r.off.assign(go, go + std::max<size_t>(n - 1, 1));
+			r.shift = h_shift[g];
+			double top = -INFINITY; // bisection may leave equal values an ulp out of order
+			for (size_t i = 0; i < n; ++i) {
+				if (!std::isfinite(gd[i]) || !std::isfinite(go[i]) || !std::isfinite(gv[i]))
+					return not_converged(g);
+				top                                 = std::max(top, gv[i]);
+				eigenvalues[eoff[g] + (long long)i] = r.shift ? std::ldexp(top, -r.shift) : top;
+				if (r.shift)
+					r.scaled_values.push_back(top);
+			}
+		}
+	} else {
+		double* h_rho = pinned<double>(0, rho_elems);
+		if (!h_rho)
+			return fail(DMRGPP_OOM, "page-locked host buffer for the density matrices");
+		if ((e = cudaGetLastError())
+		    || (e = cudaMemcpyAsync(h_rho, rho, rho_elems * sizeof(double), cudaMemcpyDeviceToHost, st))
+		    || (e = cudaStreamSynchronize(st)))
+			return cuda_fail(e, "density matrices");
+		g_trunc_times[DMRGPP_TRUNC_RHO] = seconds_since(t_start);
+		tp                              = Clock::now();
+		std::vector<double*> ga(ng), gw(ng);
+		for (size_t g = 0; g < ng; ++g) {
+			ga[g] = h_rho + goff[g];
+			gw[g] = eigenvalues + eoff[g];
+		}
+		if (!group_eigenvalues(ng, d->group_size, ga.data(), gw.data(), ge, hw)) {
+			size_t g = 0;
+			while (g < ng && ge[g].ok)
+				++g;
+			return not_converged(g);
+		}
 	}
 
 	g_trunc_times[DMRGPP_TRUNC_EIGENVALUES] = seconds_since(tp);
@@ -417,12 +852,12 @@ extern "C" int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, d
 		for (size_t g = 0; g < ng; ++g)
 			koff[g + 1] = koff[g] + (long long)(d->group_size[g] * kept[g]);
 		const size_t        kelems = size_t(std::max<long long>(koff[ng], 1));
-		// the packed reflectors: every group with kept states copies its whole
-		// n x n block; the rest is never read
-		double* hv = pinned<double>(1, rho_elems);
+		// the host reduction's packed reflectors: every group with kept states
+		// copies its whole n x n block; the rest is never read
+		double* hv = on_device ? nullptr : pinned<double>(1, rho_elems);
 		double* zk = pinned<double>(2, kelems);
 		double* vo = pinned<double>(3, kelems);
-		if (!hv || !zk || !vo)
+		if ((!on_device && !hv) || !zk || !vo)
 			return fail(DMRGPP_OOM, "page-locked host buffers for the eigenvectors");
 		std::vector<double> bt(size_t(std::max<long long>(eoff[ng], 1)), 0.0);
 		std::vector<const double*> gwk(ng);
@@ -432,13 +867,14 @@ extern "C" int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, d
 			gz[g]  = zk + koff[g];
 		}
 		group_eigenvectors(ng, d->group_size, kept, ge.data(), gwk.data(), gz.data(), hw);
-		parallel_for(ng, [&](size_t t) {
-			const size_t g = by_size[t];
-			if (kept[g] == 0)
-				return;
-			std::copy(ge[g].hv.begin(), ge[g].hv.end(), hv + goff[g]);
-			std::copy(ge[g].beta.begin(), ge[g].beta.end(), bt.begin() + eoff[g]);
-		});
+		if (!on_device)
+			parallel_for(ng, [&](size_t t) {
+				const size_t g = by_size[t];
+				if (kept[g] == 0)
+					return;
+				std::copy(ge[g].hv.begin(), ge[g].hv.end(), hv + goff[g]);
+				std::copy(ge[g].beta.begin(), ge[g].beta.end(), bt.begin() + eoff[g]);
+			});
 		g_trunc_times[DMRGPP_TRUNC_VECTORS_HOST] = seconds_since(tp);
 		tp                                       = Clock::now();
 		std::vector<ColumnJob> cj;
@@ -459,16 +895,21 @@ extern "C" int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, d
 				}
 			} freev { { &z, &v, &d_hv, &d_bt }, &d_cj };
 			if ((e = dev_malloc(&z, kelems * sizeof(double))) || (e = dev_malloc(&v, kelems * sizeof(double)))
-			    || (e = dev_malloc(&d_hv, rho_elems * sizeof(double))) || (e = dev_malloc(&d_bt, bt.size() * sizeof(double)))
 			    || (e = dev_malloc(&d_cj, cj.size() * sizeof(ColumnJob))))
 				return cuda_fail(e, "eigenvector allocation");
+			// the device reduction left its reflectors in rho's storage
+			if (!on_device
+			    && ((e = dev_malloc(&d_hv, rho_elems * sizeof(double))) || (e = dev_malloc(&d_bt, bt.size() * sizeof(double)))
+			        || (e = cudaMemcpyAsync(d_hv, hv, rho_elems * sizeof(double), cudaMemcpyHostToDevice, st))
+			        || (e = cudaMemcpyAsync(d_bt, bt.data(), bt.size() * sizeof(double), cudaMemcpyHostToDevice, st))))
+				return cuda_fail(e, "eigenvector set-up");
+			const double* refl = on_device ? rho : d_hv;
+			const double* rbet = on_device ? tri + 3 * std::max<size_t>(N, 1) : d_bt;
 			if ((e = cudaMemcpyAsync(z, zk, kelems * sizeof(double), cudaMemcpyHostToDevice, st))
-			    || (e = cudaMemcpyAsync(d_hv, hv, rho_elems * sizeof(double), cudaMemcpyHostToDevice, st))
-			    || (e = cudaMemcpyAsync(d_bt, bt.data(), bt.size() * sizeof(double), cudaMemcpyHostToDevice, st))
 			    || (e = cudaMemcpyAsync(d_cj, cj.data(), cj.size() * sizeof(ColumnJob), cudaMemcpyHostToDevice, st)))
 				return cuda_fail(e, "eigenvector set-up");
 			const int cgrid = int(std::min<size_t>((cj.size() + 7) / 8, 148 * 8));
-			k_back_transform<<<std::max(cgrid, 1), 256, 0, st>>>(z, v, d_hv, d_bt, d_cj, int(cj.size()));
+			k_back_transform<<<std::max(cgrid, 1), 256, 0, st>>>(z, v, refl, rbet, d_cj, int(cj.size()));
 			if ((e = cudaGetLastError())
 			    || (e = cudaMemcpyAsync(vo, v, size_t(koff[ng]) * sizeof(double), cudaMemcpyDeviceToHost, st))
 			    || (e = cudaStreamSynchronize(st)))
