@@ -65,6 +65,66 @@ __device__ __forceinline__ double block_sum(double v, double* red)
 	return s; // valid in thread 0
 }
 
+// Where a chunk kernel also finishes its sectors' sums: per sector its chunks
+// and an arrival counter (returned to zero by the block that ends the sector).
+struct SegSums {
+	const int* seg_chunk;
+	unsigned*  ctr;
+};
+
+// Called by the whole block once thread 0 has stored the chunk's partials:
+// true in the block whose chunk is the sector's last to arrive.
+__device__ __forceinline__ bool seg_last(const SegSums& g, int seg)
+{
+	__shared__ bool last;
+	if (threadIdx.x == 0) {
+		__threadfence();
+		const unsigned n = unsigned(g.seg_chunk[seg + 1] - g.seg_chunk[seg]);
+		last             = atomicAdd(&g.ctr[seg], 1u) == n - 1;
+		if (last) {
+			g.ctr[seg] = 0u;
+			__threadfence();
+		}
+	}
+	__syncthreads();
+	return last; // (a block_sum separates this from the next call)
+}
+
+// the sector's sum, as k_g_finish forms it (valid in thread 0)
+__device__ __forceinline__ double seg_total(const SegSums& g, int seg, const double* partial, double* red)
+{
+	double t = 0.0;
+	for (int ch = g.seg_chunk[seg] + threadIdx.x; ch < g.seg_chunk[seg + 1]; ch += kThreads)
+		t += __ldcg(partial + ch);
+	return block_sum(t, red);
+}
+
+// out[s] = <x, y> of every active sector.  The sums of a sector are finished by
+// the block that comes last, in k_g_finish's order: a launch of its own for
+// them costs as much as the sums (2.2 us and a gap, against 4.4).
+__global__ void __launch_bounds__(kThreads)
+k_g_dot_out(const double* __restrict__ x, const double* __restrict__ y, const Chunk* __restrict__ chunks,
+            int nch, const int* __restrict__ active, double* partial, SegSums sg, double* out, int root)
+{
+	__shared__ double red[kThreads / 32];
+	for (int ch = blockIdx.x; ch < nch; ch += gridDim.x) {
+		const Chunk c = chunks[ch];
+		if (!active[c.seg])
+			continue;
+		double s = 0.0;
+		for (int i = threadIdx.x; i < c.len; i += kThreads)
+			s += x[c.begin + i] * y[c.begin + i];
+		s = block_sum(s, red);
+		if (threadIdx.x == 0)
+			partial[ch] = s;
+		if (seg_last(sg, c.seg)) {
+			const double t = seg_total(sg, c.seg, partial, red);
+			if (threadIdx.x == 0)
+				out[c.seg] = root ? sqrt(t) : t;
+		}
+	}
+}
+
 // partial[ch] = <x, y> over chunk ch (0 for stopped sectors)
 __global__ void __launch_bounds__(kThreads)
 k_g_dot(const double* __restrict__ x, const double* __restrict__ y, const Chunk* __restrict__ chunks,
@@ -123,31 +183,36 @@ k_g_scale(const double* x, double* y, const double* __restrict__ scal,
 	}
 }
 
-// v2 -= alpha[s] v1 + beta[s] v0 (v0 may be null); partial[ch] = |v2|^2 over ch
+// v2 -= alpha[s] v1 + beta[s] v0 (v0 may be null), out[s] = |v2|, active sectors
 __global__ void __launch_bounds__(kThreads)
 k_g_update(double* __restrict__ v2, const double* __restrict__ v1, const double* __restrict__ v0,
            const double* __restrict__ alpha, const double* __restrict__ beta,
            const Chunk* __restrict__ chunks, int nch, const int* __restrict__ active,
-           double* __restrict__ partial)
+           double* partial, SegSums sg, double* out)
 {
 	__shared__ double red[kThreads / 32];
 	for (int ch = blockIdx.x; ch < nch; ch += gridDim.x) {
 		const Chunk c = chunks[ch];
-		double      s = 0.0;
-		if (active[c.seg]) {
-			const double a = alpha[c.seg], b = v0 ? beta[c.seg] : 0.0;
-			for (int i = threadIdx.x; i < c.len; i += kThreads) {
-				const long long q = c.begin + i;
-				double          w = v2[q] - a * v1[q];
-				if (v0)
-					w -= b * v0[q];
-				v2[q] = w;
-				s += w * w;
-			}
+		if (!active[c.seg])
+			continue;
+		double       s = 0.0;
+		const double a = alpha[c.seg], b = v0 ? beta[c.seg] : 0.0;
+		for (int i = threadIdx.x; i < c.len; i += kThreads) {
+			const long long q = c.begin + i;
+			double          w = v2[q] - a * v1[q];
+			if (v0)
+				w -= b * v0[q];
+			v2[q] = w;
+			s += w * w;
 		}
 		s = block_sum(s, red);
 		if (threadIdx.x == 0)
 			partial[ch] = s;
+		if (seg_last(sg, c.seg)) {
+			const double t = seg_total(sg, c.seg, partial, red);
+			if (threadIdx.x == 0)
+				out[c.seg] = sqrt(t);
+		}
 	}
 }
 
@@ -366,36 +431,6 @@ k_g_residual(const double* __restrict__ hu, const double* __restrict__ u, const 
 	}
 }
 
-// CG step of every active sector: alpha = rr / pAp (0 when pAp <= 0: the
-// check below then stops the sector), t += alpha p, res -= alpha Aq;
-// partial[ch] = |res|^2 over ch
-__global__ void __launch_bounds__(kThreads)
-k_g_cg_update(double* __restrict__ t, double* __restrict__ res, const double* __restrict__ p,
-              const double* __restrict__ Aq, const double* __restrict__ rr, const double* __restrict__ pAp,
-              const Chunk* __restrict__ chunks, int nch, const int* __restrict__ active,
-              double* __restrict__ partial)
-{
-	__shared__ double red[kThreads / 32];
-	for (int ch = blockIdx.x; ch < nch; ch += gridDim.x) {
-		const Chunk k = chunks[ch];
-		double      s = 0.0;
-		if (active[k.seg]) {
-			const double d     = pAp[k.seg];
-			const double alpha = d > 0.0 ? rr[k.seg] / d : 0.0;
-			for (int i = threadIdx.x; i < k.len; i += kThreads) {
-				const long long q = k.begin + i;
-				t[q] += alpha * p[q];
-				const double w = res[q] - alpha * Aq[q];
-				res[q]         = w;
-				s += w * w;
-			}
-		}
-		s = block_sum(s, red);
-		if (threadIdx.x == 0)
-			partial[ch] = s;
-	}
-}
-
 // ---- diagonal (Jacobi) preconditioner of the group correction solves, per
 // sector as in lanczos.cu (pcg_correction): K = diag(H) - theta[sector], kept
 // at least 1e-3 max(1, |theta|); z = K^-1 res - a K^-1 u with a = <u, K^-1 res>
@@ -405,6 +440,146 @@ __device__ __forceinline__ double g_pcg_k(double d, double th)
 	const double f = 1e-3 * fmax(1.0, fabs(th));
 	const double k = d - th;
 	return k > f ? k : f;
+}
+
+// One CG iteration of every active sector after Aq = H p is four launches (A to
+// C here and the direction), every sum finished in the kernel that forms it;
+// as twelve, axpys and sums apart, it took as long as the H*x itself (80 us of
+// 164 on 24 sectors).  The arithmetic and its order are those of the separate
+// steps.
+
+// A: ua = <u, Aq - theta p>
+__global__ void __launch_bounds__(kThreads)
+k_g_cg_project(const double* __restrict__ Aq, const double* __restrict__ p, const double* __restrict__ u,
+               const double* __restrict__ theta, const Chunk* __restrict__ chunks, int nch,
+               const int* __restrict__ active, double* partial, SegSums sg, double* ua)
+{
+	__shared__ double red[kThreads / 32];
+	for (int ch = blockIdx.x; ch < nch; ch += gridDim.x) {
+		const Chunk k = chunks[ch];
+		if (!active[k.seg])
+			continue;
+		const double f = -theta[k.seg];
+		double       s = 0.0;
+		for (int i = threadIdx.x; i < k.len; i += kThreads) {
+			const long long q = k.begin + i;
+			s += u[q] * (Aq[q] + f * p[q]);
+		}
+		s = block_sum(s, red);
+		if (threadIdx.x == 0)
+			partial[ch] = s;
+		if (seg_last(sg, k.seg)) {
+			const double t = seg_total(sg, k.seg, partial, red);
+			if (threadIdx.x == 0)
+				ua[k.seg] = t;
+		}
+	}
+}
+
+// B: Aq <- Aq - theta p - ua u, pAp = <p, Aq>
+__global__ void __launch_bounds__(kThreads)
+k_g_cg_curvature(double* __restrict__ Aq, const double* __restrict__ p, const double* __restrict__ u,
+                 const double* __restrict__ theta, const double* __restrict__ ua, const Chunk* __restrict__ chunks,
+                 int nch, const int* __restrict__ active, double* partial, SegSums sg, double* pAp)
+{
+	__shared__ double red[kThreads / 32];
+	for (int ch = blockIdx.x; ch < nch; ch += gridDim.x) {
+		const Chunk k = chunks[ch];
+		if (!active[k.seg])
+			continue;
+		const double f = -theta[k.seg], g = -ua[k.seg];
+		double       s = 0.0;
+		for (int i = threadIdx.x; i < k.len; i += kThreads) {
+			const long long q = k.begin + i;
+			double          v = Aq[q] + f * p[q];
+			v += g * u[q];
+			Aq[q] = v;
+			s += p[q] * v;
+		}
+		s = block_sum(s, red);
+		if (threadIdx.x == 0)
+			partial[ch] = s;
+		if (seg_last(sg, k.seg)) {
+			const double t = seg_total(sg, k.seg, partial, red);
+			if (threadIdx.x == 0)
+				pAp[k.seg] = t;
+		}
+	}
+}
+
+// C: alpha = rr / pAp (0 when pAp <= 0), t += alpha p, res -= alpha Aq, rr_next
+// = |res|^2; the sector stops on a non-positive pAp or once |res| <= tol b0.
+// With a diagonal (jac) also sums = <u, K^-1 res>, <res, K^-1 res>, <res, wv>
+// (3 x nseg) of the sectors that go on; partial holds 4 x nch.
+struct CgUpdate {
+	double *      t, *res;
+	const double *p, *Aq, *rr, *pAp;
+	double*       rr_next;
+	const double* b0;
+	double        tol;
+	const double *diag, *theta, *u, *wv; // diag NULL: no preconditioner
+	double*       sums;
+};
+
+__global__ void __launch_bounds__(kThreads)
+k_g_cg_update(const CgUpdate a, const Chunk* __restrict__ chunks, int nch, int nseg, int* active,
+              double* partial, SegSums sg)
+{
+	__shared__ double red[kThreads / 32];
+	__shared__ bool   stop;
+	for (int ch = blockIdx.x; ch < nch; ch += gridDim.x) {
+		const Chunk k = chunks[ch];
+		if (!active[k.seg])
+			continue;
+		const double d     = a.pAp[k.seg];
+		const double alpha = d > 0.0 ? a.rr[k.seg] / d : 0.0;
+		const double th    = a.diag ? a.theta[k.seg] : 0.0;
+		double       s = 0.0, v0 = 0.0, v1 = 0.0, v2 = 0.0;
+		for (int i = threadIdx.x; i < k.len; i += kThreads) {
+			const long long q = k.begin + i;
+			a.t[q] += alpha * a.p[q];
+			const double w = a.res[q] - alpha * a.Aq[q];
+			a.res[q]       = w;
+			s += w * w;
+			if (a.diag) {
+				const double z = w / g_pcg_k(a.diag[q], th);
+				v0 += a.u[q] * z;
+				v1 += w * z;
+				v2 += w * a.wv[q];
+			}
+		}
+		s = block_sum(s, red);
+		if (a.diag) {
+			v0 = block_sum(v0, red);
+			v1 = block_sum(v1, red);
+			v2 = block_sum(v2, red);
+		}
+		if (threadIdx.x == 0) {
+			partial[ch] = s;
+			if (a.diag) {
+				partial[nch + ch]     = v0;
+				partial[2 * nch + ch] = v1;
+				partial[3 * nch + ch] = v2;
+			}
+		}
+		if (!seg_last(sg, k.seg))
+			continue;
+		const double rn = seg_total(sg, k.seg, partial, red);
+		if (threadIdx.x == 0) {
+			a.rr_next[k.seg] = rn;
+			stop             = !(d > 0.0) || sqrt(rn) <= a.tol * a.b0[k.seg];
+			if (stop)
+				active[k.seg] = 0;
+		}
+		__syncthreads();
+		if (stop || !a.diag)
+			continue;
+		for (int e = 0; e < 3; ++e) {
+			const double t = seg_total(sg, k.seg, partial + size_t(e + 1) * nch, red);
+			if (threadIdx.x == 0)
+				a.sums[size_t(e) * nseg + k.seg] = t;
+		}
+	}
 }
 
 // wv = K^-1 u; partial[ch] = <u, wv> over ch
@@ -493,18 +668,6 @@ k_g_pcg_direction(double* __restrict__ p, const double* __restrict__ res, const 
 	}
 }
 
-// one thread per sector: stop the sector's CG on a non-positive pAp or once
-// |res| <= tol * b0
-__global__ void k_g_cg_check(const double* __restrict__ pAp, const double* __restrict__ rr_next,
-                             const double* __restrict__ b0, double tol, int* __restrict__ active, int nseg)
-{
-	const int s = blockIdx.x * blockDim.x + threadIdx.x;
-	if (s >= nseg || !active[s])
-		return;
-	if (!(pAp[s] > 0.0) || sqrt(rr_next[s]) <= tol * b0[s])
-		active[s] = 0;
-}
-
 // one thread per sector: the CG runs for outer-active sectors with b0 > 0
 __global__ void k_g_cg_start(const double* __restrict__ b0, const int* __restrict__ outer,
                              int* __restrict__ active, int nseg)
@@ -580,7 +743,8 @@ struct GroupWork {
 	double* rv    = nullptr; // 7 x dim: H psi, r, t, res, p, Aq, K^-1 psi (Jacobi corrections)
 	double* rsc   = nullptr; // 8 x nseg scalars
 	double* rpsc  = nullptr; // 6 x nseg: Jacobi corrections' <u,K^-1 u>, three sums, rho[2]
-	double* rpart = nullptr; // 3 x nch chunk partials of those sums
+	double* rpart = nullptr; // 4 x nch chunk partials of those sums and |res|^2
+	unsigned* segctr = nullptr; // per sector: chunks arrived (SegSums)
 	int*    rint  = nullptr; // 2 x nseg: outer active, CG active
 	double* rhost = nullptr; // pinned: theta, |r| (2 x nseg), then 2 x nseg ints
 	long long* sec_start = nullptr; // nseg + 1 sector offsets
@@ -615,6 +779,7 @@ void release_group(dmrgpp_kron_handle h)
 	dmrgpp::dev_free(w->rsc);
 	dmrgpp::dev_free(w->rpsc);
 	dmrgpp::dev_free(w->rpart);
+	dmrgpp::dev_free(w->segctr);
 	dmrgpp::dev_free(w->rint);
 	if (w->rhost)
 		cudaFreeHost(w->rhost);
@@ -668,6 +833,7 @@ int ensure_group_work(dmrgpp_kron_handle h, int cols)
 	    || (e = dmrgpp::dev_malloc(&w->chunks, std::max<size_t>(1, ch.size()) * sizeof(Chunk)))
 	    || (e = dmrgpp::dev_malloc(&w->seg_chunk, sc.size() * sizeof(int)))
 	    || (e = dmrgpp::dev_malloc(&w->active, size_t(nseg) * sizeof(int)))
+	    || (e = dmrgpp::dev_malloc(&w->segctr, size_t(nseg) * sizeof(unsigned)))
 	    || (e = dmrgpp::dev_malloc(&w->ncols, size_t(nseg) * sizeof(int)))
 	    || (e = dmrgpp::dev_malloc(&w->sec_start, (size_t(nseg) + 1) * sizeof(long long)))
 	    || (e = cudaHostAlloc(&w->host, 2 * (2 * nsc + size_t(nseg)) * sizeof(double), 0)))
@@ -677,6 +843,7 @@ int ensure_group_work(dmrgpp_kron_handle h, int cols)
 	    || (e = dmrgpp::upload_sync(w->sec_start, h->sector_start.data(), (size_t(nseg) + 1) * sizeof(long long),
 	                                h->stream))
 	    || (e = dmrgpp::clear_async(w->beta, (nsc + size_t(nseg)) * sizeof(double), h->stream))
+	    || (e = dmrgpp::clear_async(w->segctr, size_t(nseg) * sizeof(unsigned), h->stream))
 	    || (e = dmrgpp::clear_async(w->alpha, nsc * sizeof(double), h->stream)))
 		return status(h, e, "group solver set-up");
 	return DMRGPP_OK;
@@ -774,9 +941,9 @@ extern "C" int dmrgpp_lanczos_lowest_group_masked(dmrgpp_kron_handle h, const dm
 		return status(h, e, "copy initial vectors");
 
 	// per-sector reductions: partial per chunk, then one sum per sector
+	const SegSums sg { w->seg_chunk, w->segctr };
 	auto dot = [&](const double* x, const double* y, double* out, int root) {
-		k_g_dot<<<grid, kThreads, 0, st>>>(x, y, w->chunks, nch, w->active, w->partial);
-		k_g_finish<<<S, kThreads, 0, st>>>(w->partial, w->seg_chunk, w->active, out, root);
+		k_g_dot_out<<<grid, kThreads, 0, st>>>(x, y, w->chunks, nch, w->active, w->partial, sg, out, root);
 	};
 	// V0 = init / |init| per sector (LanczosCore.h:166-175)
 	dot(col(1), col(1), nrm, 0);
@@ -786,8 +953,7 @@ extern "C" int dmrgpp_lanczos_lowest_group_masked(dmrgpp_kron_handle h, const dm
 		return rc;
 	dot(col(1), col(0), al(0), 0);
 	k_g_update<<<grid, kThreads, 0, st>>>(col(1), col(0), nullptr, al(0), be(0), w->chunks, nch,
-	                                      w->active, w->partial);
-	k_g_finish<<<S, kThreads, 0, st>>>(w->partial, w->seg_chunk, w->active, be(1), 1);
+	                                      w->active, w->partial, sg, be(1));
 	k_g_scale<<<grid, kThreads, 0, st>>>(col(1), col(1), be(1), 1, w->chunks, nch, w->active);
 
 	std::vector<size_t> j_stop(size_t(S), 0);
@@ -813,8 +979,7 @@ extern "C" int dmrgpp_lanczos_lowest_group_masked(dmrgpp_kron_handle h, const dm
 				return rc;
 			dot(v2, v1, al(jj), 0);
 			k_g_update<<<grid, kThreads, 0, st>>>(v2, v1, v0, al(jj), be(jj), w->chunks, nch,
-			                                      w->active, w->partial);
-			k_g_finish<<<S, kThreads, 0, st>>>(w->partial, w->seg_chunk, w->active, be(jj + 1), 1);
+			                                      w->active, w->partial, sg, be(jj + 1));
 			k_g_scale<<<grid, kThreads, 0, st>>>(v2, v2, be(jj + 1), 1, w->chunks, nch, w->active);
 			if (p->reortho) { // reorthoIfNecessary (LanczosVectors.h:243-271)
 				const int nc = int(jj) + 1;
@@ -1029,7 +1194,7 @@ extern "C" int dmrgpp_refine_lowest_group(dmrgpp_kron_handle h, double* psi, int
 		if ((e = dmrgpp::dev_malloc(&w->rv, 7 * D * sizeof(double)))
 		    || (e = dmrgpp::dev_malloc(&w->rsc, 8 * size_t(S) * sizeof(double)))
 		    || (e = dmrgpp::dev_malloc(&w->rpsc, 6 * size_t(S) * sizeof(double)))
-		    || (e = dmrgpp::dev_malloc(&w->rpart, 3 * size_t(std::max(w->nch, 1)) * sizeof(double)))
+		    || (e = dmrgpp::dev_malloc(&w->rpart, 4 * size_t(std::max(w->nch, 1)) * sizeof(double)))
 		    || (e = dmrgpp::dev_malloc(&w->rint, 2 * size_t(S) * sizeof(int)))
 		    || (e = cudaHostAlloc(&w->rhost, 2 * size_t(S) * (sizeof(double) + sizeof(int)), 0)))
 			return status(h, e, "group refinement allocation");
@@ -1056,9 +1221,9 @@ extern "C" int dmrgpp_refine_lowest_group(dmrgpp_kron_handle h, double* psi, int
 	double*   rn_h  = w->rhost + S;
 	int*      cg_h  = reinterpret_cast<int*>(w->rhost + 2 * S);
 
+	const SegSums sg { w->seg_chunk, w->segctr };
 	auto dot = [&](const double* x, const double* y, double* out, const int* act, int root) {
-		k_g_dot<<<grid, kThreads, 0, st>>>(x, y, w->chunks, nch, act, w->partial);
-		k_g_finish<<<S, kThreads, 0, st>>>(w->partial, w->seg_chunk, act, out, root);
+		k_g_dot_out<<<grid, kThreads, 0, st>>>(x, y, w->chunks, nch, act, w->partial, sg, out, root);
 	};
 	// Jacobi corrections (dmrgpp_set_correction_preconditioner)
 	const bool jac  = h->correction_precond == DMRGPP_PRECOND_JACOBI && h->d_diag;
@@ -1173,17 +1338,14 @@ extern "C" int dmrgpp_refine_lowest_group(dmrgpp_kron_handle h, double* psi, int
 				if (rc)
 					return rc;
 				++s.inner_matvecs;
-				k_g_axpy<<<grid, kThreads, 0, st>>>(Aq, pv, theta, -1.0, w->chunks, nch, cg);
-				dot(psi, Aq, ua, cg, 0);
-				k_g_axpy<<<grid, kThreads, 0, st>>>(Aq, psi, ua, -1.0, w->chunks, nch, cg);
-				dot(pv, Aq, pAp, cg, 0);
+				k_g_cg_project<<<grid, kThreads, 0, st>>>(Aq, pv, psi, theta, w->chunks, nch, cg, w->rpart, sg, ua);
+				k_g_cg_curvature<<<grid, kThreads, 0, st>>>(Aq, pv, psi, theta, ua, w->chunks, nch, cg, w->rpart, sg,
+				                                            pAp);
 				// alpha = rr / pAp (plain) or rho / pAp (Jacobi); |res|^2 for the check
-				k_g_cg_update<<<grid, kThreads, 0, st>>>(t, res, pv, Aq, jac ? rho[cur] : rr[cur], pAp,
-				                                         w->chunks, nch, cg, w->partial);
-				k_g_finish<<<S, kThreads, 0, st>>>(w->partial, w->seg_chunk, cg, rr[cur ^ 1], 0);
-				k_g_cg_check<<<sgrid, kThreads, 0, st>>>(pAp, rr[cur ^ 1], b0, inner_tolerance, cg, S);
+				const CgUpdate up { t,  res,      pv,    Aq,  jac ? rho[cur] : rr[cur], pAp, rr[cur ^ 1], b0, inner_tolerance,
+					            jac ? h->d_diag : nullptr, theta, psi, wv, sums };
+				k_g_cg_update<<<grid, kThreads, 0, st>>>(up, w->chunks, nch, S, cg, w->rpart, sg);
 				if (jac) {
-					pcg_sums();
 					k_g_pcg_direction<<<grid, kThreads, 0, st>>>(pv, res, h->d_diag, theta, wv, uw, sums, S,
 					                                             rho[cur], rho[cur ^ 1], 0, w->chunks, nch,
 					                                             w->seg_chunk, cg);
@@ -1329,9 +1491,9 @@ extern "C" int dmrgpp_davidson_lowest_group(dmrgpp_kron_handle h, const dmrgpp_d
 	const bool          mixed    = h->precision != DMRGPP_FP64;
 	int                 n_active = S;
 	int                 k        = 0;
+	const SegSums sg { w->seg_chunk, w->segctr };
 	auto dot = [&](const double* x, const double* y, double* out) {
-		k_g_dot<<<grid, kThreads, 0, st>>>(x, y, w->chunks, nch, w->active, w->partial);
-		k_g_finish<<<S, kThreads, 0, st>>>(w->partial, w->seg_chunk, w->active, out, 0);
+		k_g_dot_out<<<grid, kThreads, 0, st>>>(x, y, w->chunks, nch, w->active, w->partial, sg, out, 0);
 	};
 	for (size_t it = 0; it < p->max_iterations && n_active > 0; ++it) {
 		// orthonormalise the corrections against the bases and append them

@@ -1355,6 +1355,42 @@ k_axpy_neg_dev(const double* a, const double* __restrict__ x, double* __restrict
 		y[i] -= c * x[i];
 }
 
+// *ua = <u, Aq - theta p>: the first half of Aq <- P (H - theta) p, Aq = H p,
+// without writing it (the axpy and the sum as one launch and one pass; the
+// second half writes)
+__global__ void __launch_bounds__(kThreads)
+k_cg_project(const double* __restrict__ Aq, const double* __restrict__ p, const double* __restrict__ u,
+             double theta, size_t n, double* ua, double* partial, unsigned* ctr)
+{
+	__shared__ double red[kThreads / 32];
+	const double      f = -theta;
+	double            s = 0.0;
+	for (size_t i = blockIdx.x * size_t(kThreads) + threadIdx.x; i < n;
+	     i += size_t(gridDim.x) * kThreads)
+		s += u[i] * (Aq[i] + f * p[i]);
+	s = block_sum(s, red);
+	grid_sum(s, partial, ctr, ua, false, red);
+}
+
+// Aq <- Aq - theta p - *ua u, *pAp = <p, Aq>
+__global__ void __launch_bounds__(kThreads)
+k_cg_curvature(double* __restrict__ Aq, const double* __restrict__ p, const double* __restrict__ u,
+               double theta, const double* ua, size_t n, double* pAp, double* partial, unsigned* ctr)
+{
+	__shared__ double red[kThreads / 32];
+	const double      f = -theta, c = *ua;
+	double            s = 0.0;
+	for (size_t i = blockIdx.x * size_t(kThreads) + threadIdx.x; i < n;
+	     i += size_t(gridDim.x) * kThreads) {
+		double v = Aq[i] + f * p[i];
+		v -= c * u[i];
+		Aq[i] = v;
+		s += p[i] * v;
+	}
+	s = block_sum(s, red);
+	grid_sum(s, partial, ctr, pAp, false, red);
+}
+
 // conjugate-gradient update with device scalars: alpha = rr / pAp;
 // t += alpha p; res -= alpha Aq; *rr_next = |res|^2.  A non-positive pAp (or
 // an earlier one, *broken) freezes the iteration: alpha = 0 and *broken = 1.
@@ -1451,6 +1487,18 @@ __device__ __forceinline__ void grid_sum4(double (&v)[4], double* partial, unsig
 	}
 }
 
+// element i of the sums <u, K^-1 res>, <res, K^-1 res>, <res, wv>, <res, res>
+__device__ __forceinline__ void pcg_add(double (&v)[4], double r, size_t i, const double* __restrict__ diag,
+                                        double theta, double floor_, const double* __restrict__ u,
+                                        const double* __restrict__ wv)
+{
+	const double z = r / pcg_k(diag[i], theta, floor_);
+	v[0] += u[i] * z;
+	v[1] += r * z;
+	v[2] += r * wv[i];
+	v[3] += r * r;
+}
+
 // sums = <u, K^-1 res>, <res, K^-1 res>, <res, wv>, <res, res>
 __device__ __forceinline__ void pcg_sums_body(const double* __restrict__ res, const double* __restrict__ diag,
                                               double theta, double floor_, const double* __restrict__ u,
@@ -1459,14 +1507,8 @@ __device__ __forceinline__ void pcg_sums_body(const double* __restrict__ res, co
 {
 	double v[4] = { 0.0, 0.0, 0.0, 0.0 };
 	for (size_t i = blockIdx.x * size_t(kThreads) + threadIdx.x; i < n;
-	     i += size_t(gridDim.x) * kThreads) {
-		const double r = res[i];
-		const double z = r / pcg_k(diag[i], theta, floor_);
-		v[0] += u[i] * z;
-		v[1] += r * z;
-		v[2] += r * wv[i];
-		v[3] += r * r;
-	}
+	     i += size_t(gridDim.x) * kThreads)
+		pcg_add(v, res[i], i, diag, theta, floor_, u, wv);
 	grid_sum4(v, partial, ctr, sums, red);
 }
 
@@ -1493,13 +1535,15 @@ k_pcg_update(double* __restrict__ t, double* __restrict__ res, const double* __r
 	const double      alpha = stop ? 0.0 : *rho / *pAp;
 	if (stop && blockIdx.x == 0 && threadIdx.x == 0)
 		*broken = 1.0;
+	double v[4] = { 0.0, 0.0, 0.0, 0.0 };
 	for (size_t i = blockIdx.x * size_t(kThreads) + threadIdx.x; i < n;
 	     i += size_t(gridDim.x) * kThreads) {
 		t[i] += alpha * p[i];
-		res[i] -= alpha * Aq[i];
+		const double r = res[i] - alpha * Aq[i];
+		res[i]         = r;
+		pcg_add(v, r, i, diag, theta, floor_, u, wv);
 	}
-	// each thread re-reads only the elements it wrote: no grid barrier needed
-	pcg_sums_body(res, diag, theta, floor_, u, wv, n, sums, partial, ctr, red);
+	grid_sum4(v, partial, ctr, sums, red);
 }
 
 // z = K^-1 res - a wv with a = sums[0] / *uw; rho_new = sums[1] - a sums[2];
@@ -1572,10 +1616,8 @@ int pcg_correction(dmrgpp_kron_handle h, const double* u, double theta, const do
 			// Aq = P (H - theta) p  (p orthogonal to u up to round-off)
 			if (int rc = kron_apply_device(h, p, Aq))
 				return rc;
-			k_axpy<<<nb, kThreads, 0, st>>>(-theta, p, Aq, D);
-			k_dot<<<nb, kThreads, 0, st>>>(u, Aq, D, sc + 0, w->partial, w->ctr + 5);
-			k_axpy_neg_dev<<<nb, kThreads, 0, st>>>(sc + 0, u, Aq, D);
-			k_dot<<<nb, kThreads, 0, st>>>(p, Aq, D, sc + 1, w->partial, w->ctr + 7);
+			k_cg_project<<<nb, kThreads, 0, st>>>(Aq, p, u, theta, D, sc + 0, w->partial, w->ctr + 5);
+			k_cg_curvature<<<nb, kThreads, 0, st>>>(Aq, p, u, theta, sc + 0, D, sc + 1, w->partial, w->ctr + 7);
 			k_pcg_update<<<nb, kThreads, 0, st>>>(t, res, p, Aq, sc + 10 + cur, sc + 1, sc + 4, h->d_diag,
 			                                      theta, floor_, u, wv, D, sc + 6, w->partial, w->ctr + 9);
 			k_pcg_direction<<<nb, kThreads, 0, st>>>(p, res, h->d_diag, theta, floor_, wv, sc + 5, sc + 6,
@@ -1681,10 +1723,8 @@ int dmrgpp_correction_solve(dmrgpp_kron_handle h, const double* u, double theta,
 			// Aq = P (H - theta) p  (p orthogonal to u up to round-off)
 			if (int rc = kron_apply_device(h, p, Aq))
 				return rc;
-			k_axpy<<<nb, kThreads, 0, st>>>(-theta, p, Aq, D);
-			k_dot<<<nb, kThreads, 0, st>>>(u, Aq, D, sc + 0, w->partial, w->ctr + 5);
-			k_axpy_neg_dev<<<nb, kThreads, 0, st>>>(sc + 0, u, Aq, D);
-			k_dot<<<nb, kThreads, 0, st>>>(p, Aq, D, sc + 1, w->partial, w->ctr + 7);
+			k_cg_project<<<nb, kThreads, 0, st>>>(Aq, p, u, theta, D, sc + 0, w->partial, w->ctr + 5);
+			k_cg_curvature<<<nb, kThreads, 0, st>>>(Aq, p, u, theta, sc + 0, D, sc + 1, w->partial, w->ctr + 7);
 			k_cg_update<<<nb, kThreads, 0, st>>>(t, res, p, Aq, sc + 2 + cur, sc + 1, sc + 3 - cur,
 			                                     sc + 4, D, w->partial, w->ctr + 6);
 			k_cg_direction<<<nb, kThreads, 0, st>>>(p, res, sc + 3 - cur, sc + 2 + cur, sc + 4, D);
