@@ -65,6 +65,29 @@ __device__ __forceinline__ double block_sum(double v, double* red)
 	return s; // valid in thread 0
 }
 
+// four block_sums at once (each in block_sum's order): v[q] valid in thread q
+__device__ __forceinline__ double block_sum4(const double (&v)[4], double (*red)[kThreads / 32])
+{
+	double t[4];
+#pragma unroll
+	for (int q = 0; q < 4; ++q) {
+		t[q] = v[q];
+		for (int o = 16; o > 0; o >>= 1)
+			t[q] += __shfl_down_sync(0xffffffffu, t[q], o);
+	}
+	if ((threadIdx.x & 31) == 0)
+#pragma unroll
+		for (int q = 0; q < 4; ++q)
+			red[q][threadIdx.x >> 5] = t[q];
+	__syncthreads();
+	double s = 0.0;
+	if (threadIdx.x < 4)
+		for (int w = 0; w < kThreads / 32; ++w)
+			s += red[threadIdx.x][w];
+	__syncthreads();
+	return s;
+}
+
 // Where a chunk kernel also finishes its sectors' sums: per sector its chunks
 // and an arrival counter (returned to zero by the block that ends the sector).
 struct SegSums {
@@ -525,7 +548,7 @@ __global__ void __launch_bounds__(kThreads)
 k_g_cg_update(const CgUpdate a, const Chunk* __restrict__ chunks, int nch, int nseg, int* active,
               double* partial, SegSums sg)
 {
-	__shared__ double red[kThreads / 32];
+	__shared__ double red[4][kThreads / 32];
 	__shared__ bool   stop;
 	for (int ch = blockIdx.x; ch < nch; ch += gridDim.x) {
 		const Chunk k = chunks[ch];
@@ -534,51 +557,44 @@ k_g_cg_update(const CgUpdate a, const Chunk* __restrict__ chunks, int nch, int n
 		const double d     = a.pAp[k.seg];
 		const double alpha = d > 0.0 ? a.rr[k.seg] / d : 0.0;
 		const double th    = a.diag ? a.theta[k.seg] : 0.0;
-		double       s = 0.0, v0 = 0.0, v1 = 0.0, v2 = 0.0;
+		double       v[4]  = { 0.0, 0.0, 0.0, 0.0 };
 		for (int i = threadIdx.x; i < k.len; i += kThreads) {
 			const long long q = k.begin + i;
 			a.t[q] += alpha * a.p[q];
 			const double w = a.res[q] - alpha * a.Aq[q];
 			a.res[q]       = w;
-			s += w * w;
+			v[0] += w * w;
 			if (a.diag) {
 				const double z = w / g_pcg_k(a.diag[q], th);
-				v0 += a.u[q] * z;
-				v1 += w * z;
-				v2 += w * a.wv[q];
+				v[1] += a.u[q] * z;
+				v[2] += w * z;
+				v[3] += w * a.wv[q];
 			}
 		}
-		s = block_sum(s, red);
-		if (a.diag) {
-			v0 = block_sum(v0, red);
-			v1 = block_sum(v1, red);
-			v2 = block_sum(v2, red);
+		double s = block_sum4(v, red);
+		if (threadIdx.x < 4) {
+			partial[threadIdx.x * nch + ch] = s;
+			__threadfence();
 		}
-		if (threadIdx.x == 0) {
-			partial[ch] = s;
-			if (a.diag) {
-				partial[nch + ch]     = v0;
-				partial[2 * nch + ch] = v1;
-				partial[3 * nch + ch] = v2;
-			}
-		}
+		__syncthreads(); // all four are out before thread 0 reports the chunk
 		if (!seg_last(sg, k.seg))
 			continue;
-		const double rn = seg_total(sg, k.seg, partial, red);
+#pragma unroll
+		for (int e = 0; e < 4; ++e) {
+			v[e] = 0.0;
+			for (int c = sg.seg_chunk[k.seg] + threadIdx.x; c < sg.seg_chunk[k.seg + 1]; c += kThreads)
+				v[e] += __ldcg(partial + size_t(e) * nch + c);
+		}
+		s = block_sum4(v, red);
 		if (threadIdx.x == 0) {
-			a.rr_next[k.seg] = rn;
-			stop             = !(d > 0.0) || sqrt(rn) <= a.tol * a.b0[k.seg];
+			a.rr_next[k.seg] = s;
+			stop             = !(d > 0.0) || sqrt(s) <= a.tol * a.b0[k.seg];
 			if (stop)
 				active[k.seg] = 0;
 		}
 		__syncthreads();
-		if (stop || !a.diag)
-			continue;
-		for (int e = 0; e < 3; ++e) {
-			const double t = seg_total(sg, k.seg, partial + size_t(e + 1) * nch, red);
-			if (threadIdx.x == 0)
-				a.sums[size_t(e) * nseg + k.seg] = t;
-		}
+		if (!stop && a.diag && threadIdx.x >= 1 && threadIdx.x < 4)
+			a.sums[size_t(threadIdx.x - 1) * nseg + k.seg] = s;
 	}
 }
 

@@ -1459,32 +1459,48 @@ k_pcg_setup(const double* __restrict__ u, const double* __restrict__ diag, doubl
 
 // four sums at once (deterministic: per-block partials in 4 strided slots,
 // the last block adds them in block order): sums[0..3]
-__device__ __forceinline__ void grid_sum4(double (&v)[4], double* partial, unsigned* ctr, double* sums,
-                                          double* red)
+__device__ __forceinline__ void grid_sum4(double (&v)[4], double* partial, unsigned* ctr, double* sums)
 {
-	__shared__ bool last;
-	double          b[4];
+	__shared__ bool   last;
+	__shared__ double red4[4][kThreads / 32];
+	// four block_sums at once, each in block_sum's order: value q in thread q
+	auto sum4 = [&](const double (&x)[4]) {
 #pragma unroll
-	for (int q = 0; q < 4; ++q)
-		b[q] = block_sum(v[q], red);
-	if (threadIdx.x == 0) {
-#pragma unroll
-		for (int q = 0; q < 4; ++q)
-			partial[size_t(q) * gridDim.x + blockIdx.x] = b[q];
-		last = last_block(ctr);
+		for (int q = 0; q < 4; ++q) {
+			double t = x[q];
+			for (int o = 16; o > 0; o >>= 1)
+				t += __shfl_down_sync(0xffffffffu, t, o);
+			if ((threadIdx.x & 31) == 0)
+				red4[q][threadIdx.x >> 5] = t;
+		}
+		__syncthreads();
+		double s = 0.0;
+		if (threadIdx.x < 4)
+			for (int w = 0; w < kThreads / 32; ++w)
+				s += red4[threadIdx.x][w];
+		__syncthreads();
+		return s;
+	};
+	double s = sum4(v);
+	if (threadIdx.x < 4) {
+		partial[size_t(threadIdx.x) * gridDim.x + blockIdx.x] = s;
+		__threadfence();
 	}
+	__syncthreads(); // all four are out before thread 0 reports the block
+	if (threadIdx.x == 0)
+		last = last_block(ctr);
 	__syncthreads();
 	if (!last)
 		return;
 #pragma unroll
 	for (int q = 0; q < 4; ++q) {
-		double t = 0.0;
+		v[q] = 0.0;
 		for (int k = threadIdx.x; k < int(gridDim.x); k += blockDim.x)
-			t += __ldcg(partial + size_t(q) * gridDim.x + k);
-		t = block_sum(t, red);
-		if (threadIdx.x == 0)
-			sums[q] = t;
+			v[q] += __ldcg(partial + size_t(q) * gridDim.x + k);
 	}
+	s = sum4(v);
+	if (threadIdx.x < 4)
+		sums[threadIdx.x] = s;
 }
 
 // element i of the sums <u, K^-1 res>, <res, K^-1 res>, <res, wv>, <res, res>
@@ -1503,13 +1519,13 @@ __device__ __forceinline__ void pcg_add(double (&v)[4], double r, size_t i, cons
 __device__ __forceinline__ void pcg_sums_body(const double* __restrict__ res, const double* __restrict__ diag,
                                               double theta, double floor_, const double* __restrict__ u,
                                               const double* __restrict__ wv, size_t n, double* sums,
-                                              double* partial, unsigned* ctr, double* red)
+                                              double* partial, unsigned* ctr)
 {
 	double v[4] = { 0.0, 0.0, 0.0, 0.0 };
 	for (size_t i = blockIdx.x * size_t(kThreads) + threadIdx.x; i < n;
 	     i += size_t(gridDim.x) * kThreads)
 		pcg_add(v, res[i], i, diag, theta, floor_, u, wv);
-	grid_sum4(v, partial, ctr, sums, red);
+	grid_sum4(v, partial, ctr, sums);
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -1517,8 +1533,7 @@ k_pcg_sums(const double* __restrict__ res, const double* __restrict__ diag, doub
            const double* __restrict__ u, const double* __restrict__ wv, size_t n, double* sums,
            double* partial, unsigned* ctr)
 {
-	__shared__ double red[kThreads / 32];
-	pcg_sums_body(res, diag, theta, floor_, u, wv, n, sums, partial, ctr, red);
+	pcg_sums_body(res, diag, theta, floor_, u, wv, n, sums, partial, ctr);
 }
 
 // alpha = rho / pAp; t += alpha p; res -= alpha Aq; then the four sums of the
@@ -1530,7 +1545,6 @@ k_pcg_update(double* __restrict__ t, double* __restrict__ res, const double* __r
              const double* __restrict__ diag, double theta, double floor_, const double* __restrict__ u,
              const double* __restrict__ wv, size_t n, double* sums, double* partial, unsigned* ctr)
 {
-	__shared__ double red[kThreads / 32];
 	const bool        stop  = *broken != 0.0 || !(*pAp > 0.0);
 	const double      alpha = stop ? 0.0 : *rho / *pAp;
 	if (stop && blockIdx.x == 0 && threadIdx.x == 0)
@@ -1543,7 +1557,7 @@ k_pcg_update(double* __restrict__ t, double* __restrict__ res, const double* __r
 		res[i]         = r;
 		pcg_add(v, r, i, diag, theta, floor_, u, wv);
 	}
-	grid_sum4(v, partial, ctr, sums, red);
+	grid_sum4(v, partial, ctr, sums);
 }
 
 // z = K^-1 res - a wv with a = sums[0] / *uw; rho_new = sums[1] - a sums[2];
