@@ -181,6 +181,8 @@ def nonbatched_cpu(prob, f_alg, calls=30):
     with one task thread per host core and one BLAS thread each; median of
     `calls` matvecs after one warm-up."""
     import oracle
+    if not oracle.ref_available():
+        return {"unavailable": "reference CPU build (oracle/_ref) not present"}
     x = np.random.default_rng(7).standard_normal(prob.dim)
     kc = oracle.RefKronConn(prob)
     cores = os.cpu_count() or 1
