@@ -484,6 +484,7 @@ k_g_cg_project(const double* __restrict__ Aq, const double* __restrict__ p, cons
 			continue;
 		const double f = -theta[k.seg];
 		double       s = 0.0;
+#pragma unroll 4
 		for (int i = threadIdx.x; i < k.len; i += kThreads) {
 			const long long q = k.begin + i;
 			s += u[q] * (Aq[q] + f * p[q]);
@@ -512,6 +513,7 @@ k_g_cg_curvature(double* __restrict__ Aq, const double* __restrict__ p, const do
 			continue;
 		const double f = -theta[k.seg], g = -ua[k.seg];
 		double       s = 0.0;
+#pragma unroll 4
 		for (int i = threadIdx.x; i < k.len; i += kThreads) {
 			const long long q = k.begin + i;
 			double          v = Aq[q] + f * p[q];
@@ -534,19 +536,15 @@ k_g_cg_curvature(double* __restrict__ Aq, const double* __restrict__ p, const do
 // = |res|^2; the sector stops on a non-positive pAp or once |res| <= tol b0.
 // With a diagonal (jac) also sums = <u, K^-1 res>, <res, K^-1 res>, <res, wv>
 // (3 x nseg) of the sectors that go on; partial holds 4 x nch.
-struct CgUpdate {
-	double *      t, *res;
-	const double *p, *Aq, *rr, *pAp;
-	double*       rr_next;
-	const double* b0;
-	double        tol;
-	const double *diag, *theta, *u, *wv; // diag NULL: no preconditioner
-	double*       sums;
-};
-
+// (restrict parameters: with the vectors in a struct each element's loads
+// waited for the previous one's stores)
 __global__ void __launch_bounds__(kThreads)
-k_g_cg_update(const CgUpdate a, const Chunk* __restrict__ chunks, int nch, int nseg, int* active,
-              double* partial, SegSums sg)
+k_g_cg_update(double* __restrict__ t, double* __restrict__ res, const double* __restrict__ p,
+              const double* __restrict__ Aq, const double* __restrict__ rr, const double* __restrict__ pAp,
+              double* __restrict__ rr_next, const double* __restrict__ b0, double tol,
+              const double* __restrict__ diag, const double* __restrict__ theta, const double* __restrict__ u,
+              const double* __restrict__ wv, double* __restrict__ sums, const Chunk* __restrict__ chunks, int nch,
+              int nseg, int* active, double* partial, SegSums sg)
 {
 	__shared__ double red[4][kThreads / 32];
 	__shared__ bool   stop;
@@ -554,21 +552,22 @@ k_g_cg_update(const CgUpdate a, const Chunk* __restrict__ chunks, int nch, int n
 		const Chunk k = chunks[ch];
 		if (!active[k.seg])
 			continue;
-		const double d     = a.pAp[k.seg];
-		const double alpha = d > 0.0 ? a.rr[k.seg] / d : 0.0;
-		const double th    = a.diag ? a.theta[k.seg] : 0.0;
+		const double d     = pAp[k.seg];
+		const double alpha = d > 0.0 ? rr[k.seg] / d : 0.0;
+		const double th    = diag ? theta[k.seg] : 0.0;
 		double       v[4]  = { 0.0, 0.0, 0.0, 0.0 };
+#pragma unroll 4
 		for (int i = threadIdx.x; i < k.len; i += kThreads) {
 			const long long q = k.begin + i;
-			a.t[q] += alpha * a.p[q];
-			const double w = a.res[q] - alpha * a.Aq[q];
-			a.res[q]       = w;
+			t[q] += alpha * p[q];
+			const double w = res[q] - alpha * Aq[q];
+			res[q]       = w;
 			v[0] += w * w;
-			if (a.diag) {
-				const double z = w / g_pcg_k(a.diag[q], th);
-				v[1] += a.u[q] * z;
+			if (diag) {
+				const double z = w / g_pcg_k(diag[q], th);
+				v[1] += u[q] * z;
 				v[2] += w * z;
-				v[3] += w * a.wv[q];
+				v[3] += w * wv[q];
 			}
 		}
 		double s = block_sum4(v, red);
@@ -587,14 +586,14 @@ k_g_cg_update(const CgUpdate a, const Chunk* __restrict__ chunks, int nch, int n
 		}
 		s = block_sum4(v, red);
 		if (threadIdx.x == 0) {
-			a.rr_next[k.seg] = s;
-			stop             = !(d > 0.0) || sqrt(s) <= a.tol * a.b0[k.seg];
+			rr_next[k.seg] = s;
+			stop             = !(d > 0.0) || sqrt(s) <= tol * b0[k.seg];
 			if (stop)
 				active[k.seg] = 0;
 		}
 		__syncthreads();
-		if (!stop && a.diag && threadIdx.x >= 1 && threadIdx.x < 4)
-			a.sums[size_t(threadIdx.x - 1) * nseg + k.seg] = s;
+		if (!stop && diag && threadIdx.x >= 1 && threadIdx.x < 4)
+			sums[size_t(threadIdx.x - 1) * nseg + k.seg] = s;
 	}
 }
 
@@ -676,6 +675,7 @@ k_g_pcg_direction(double* __restrict__ p, const double* __restrict__ res, const 
 		if (threadIdx.x == 0 && ch == seg_chunk[sg])
 			rho_next[sg] = rho_new;
 		const double th = theta[sg];
+#pragma unroll 4
 		for (int i = threadIdx.x; i < k.len; i += kThreads) {
 			const long long q = k.begin + i;
 			const double    z = res[q] / g_pcg_k(diag[q], th) - a * wv[q];
@@ -1358,9 +1358,9 @@ extern "C" int dmrgpp_refine_lowest_group(dmrgpp_kron_handle h, double* psi, int
 				k_g_cg_curvature<<<grid, kThreads, 0, st>>>(Aq, pv, psi, theta, ua, w->chunks, nch, cg, w->rpart, sg,
 				                                            pAp);
 				// alpha = rr / pAp (plain) or rho / pAp (Jacobi); |res|^2 for the check
-				const CgUpdate up { t,  res,      pv,    Aq,  jac ? rho[cur] : rr[cur], pAp, rr[cur ^ 1], b0, inner_tolerance,
-					            jac ? h->d_diag : nullptr, theta, psi, wv, sums };
-				k_g_cg_update<<<grid, kThreads, 0, st>>>(up, w->chunks, nch, S, cg, w->rpart, sg);
+				k_g_cg_update<<<grid, kThreads, 0, st>>>(t, res, pv, Aq, jac ? rho[cur] : rr[cur], pAp, rr[cur ^ 1],
+				                                         b0, inner_tolerance, jac ? h->d_diag : nullptr, theta, psi,
+				                                         wv, sums, w->chunks, nch, S, cg, w->rpart, sg);
 				if (jac) {
 					k_g_pcg_direction<<<grid, kThreads, 0, st>>>(pv, res, h->d_diag, theta, wv, uw, sums, S,
 					                                             rho[cur], rho[cur ^ 1], 0, w->chunks, nch,

@@ -1365,6 +1365,7 @@ k_cg_project(const double* __restrict__ Aq, const double* __restrict__ p, const 
 	__shared__ double red[kThreads / 32];
 	const double      f = -theta;
 	double            s = 0.0;
+#pragma unroll 4
 	for (size_t i = blockIdx.x * size_t(kThreads) + threadIdx.x; i < n;
 	     i += size_t(gridDim.x) * kThreads)
 		s += u[i] * (Aq[i] + f * p[i]);
@@ -1380,6 +1381,7 @@ k_cg_curvature(double* __restrict__ Aq, const double* __restrict__ p, const doub
 	__shared__ double red[kThreads / 32];
 	const double      f = -theta, c = *ua;
 	double            s = 0.0;
+#pragma unroll 4
 	for (size_t i = blockIdx.x * size_t(kThreads) + threadIdx.x; i < n;
 	     i += size_t(gridDim.x) * kThreads) {
 		double v = Aq[i] + f * p[i];
@@ -1550,6 +1552,7 @@ k_pcg_update(double* __restrict__ t, double* __restrict__ res, const double* __r
 	if (stop && blockIdx.x == 0 && threadIdx.x == 0)
 		*broken = 1.0;
 	double v[4] = { 0.0, 0.0, 0.0, 0.0 };
+#pragma unroll 4
 	for (size_t i = blockIdx.x * size_t(kThreads) + threadIdx.x; i < n;
 	     i += size_t(gridDim.x) * kThreads) {
 		t[i] += alpha * p[i];
@@ -1576,6 +1579,7 @@ k_pcg_direction(double* __restrict__ p, const double* __restrict__ res, const do
 	const double beta    = first ? 0.0 : (*rho > 0.0 ? rho_new / *rho : 0.0);
 	if (blockIdx.x == 0 && threadIdx.x == 0)
 		*rho_next = rho_new;
+#pragma unroll 4
 	for (size_t i = blockIdx.x * size_t(kThreads) + threadIdx.x; i < n;
 	     i += size_t(gridDim.x) * kThreads) {
 		const double z = res[i] / pcg_k(diag[i], theta, floor_) - a * wv[i];
