@@ -603,8 +603,24 @@ std::string validate_fused_schedule(const KronPlan& plan, int bm, int bn, int cl
 			return at("y tile out of range", q);
 		for (int u = it.u_begin; u < it.u_end; ++u) {
 			const FusedUnit& d = U[size_t(u)];
-			if (d.rj < 1 || d.cw < 1 || d.lj < d.cw || d.ldb < 1)
+			if (d.rj < 1 || d.cw < 1 || d.ldb < 1 || (d.kind == kSegXB ? d.rj : d.lj) < d.cw)
 				return at("unit shape", q);
+			if (d.kind == kSegXA) { // X rows m0.. as the A operand
+				if (!in(d.x_off + it.m0, d.x_off + (long long)(d.cw - 1) * d.rj + it.m0 + Mt - 1, dim))
+					return at("x load out of range", q);
+				if (!in(d.at_off + (long long)it.n0 * d.lj, d.at_off + (long long)(it.n0 + Nt - 1) * d.lj + d.cw - 1, ops))
+					return at("A^T load out of the operators", q);
+				continue;
+			}
+			if (d.kind == kSegXB) { // X columns n0.. as the B operand
+				if (!in(d.b_off + it.m0, d.b_off + (long long)(d.cw - 1) * d.ldb + it.m0 + Mt - 1, ops))
+					return at("B load out of the operators", q);
+				if (!in(d.x_off + (long long)it.n0 * d.rj, d.x_off + (long long)(it.n0 + Nt - 1) * d.rj + d.cw - 1, dim))
+					return at("x load out of range", q);
+				continue;
+			}
+			if (d.kind != 0)
+				return at("unit kind", q);
 			if (!in(d.b_off + it.m0, d.b_off + (long long)(d.rj - 1) * d.ldb + it.m0 + Mt - 1, ops))
 				return at("B load out of the operators", q);
 			if (!in(d.x_off, d.x_off + (long long)(d.cw - 1) * d.rj + d.rj - 1, dim))
@@ -745,6 +761,27 @@ void build_fused_schedule(KronPlan& plan, int bm, int bn, int cw, int cluster, i
 				for (size_t t = tri_begin[i]; t < tri_begin[i + 1]; ++t) {
 					const Triple&   tr = plan.triples[t];
 					const long long rj = plan.r[tr.j], lj = plan.l[tr.j];
+					const int       tk = term_kind(plan.ident[t]);
+					if (tk != 2) { // one product, cut along its contraction
+						const long long K = tk == 1 ? lj : rj;
+						for (long long c0 = 0; c0 < K; c0 += cw) {
+							FusedUnit u {};
+							u.kind   = tk == 1 ? kSegXA : kSegXB;
+							u.cw     = int(std::min<long long>(cw, K - c0));
+							u.ldb    = int(plan.M[tr.j]);
+							u.b_off  = plan.bstack_off[tr.j] + plan.row_off[t] + (tk == 1 ? 0 : c0 * u.ldb);
+							u.rj     = int(rj);
+							u.x_off  = plan.xy_start[tr.j] + (tk == 1 ? c0 * rj : c0);
+							u.at_off = plan.at_off[t] + (tk == 1 ? c0 : 0);
+							u.lj     = int(lj);
+							plan.funits.push_back(u);
+							const double k2 = double(up(u.cw, 16));
+							const double w  = 2.0 * bme * bne * k2 + step_cost * k2 / 16.0;
+							uwork.push_back(w);
+							tl.work += w;
+						}
+						continue;
+					}
 					for (long long c0 = 0; c0 < lj; c0 += cw) {
 						FusedUnit u {};
 						u.cw     = int(std::min<long long>(cw, lj - c0));

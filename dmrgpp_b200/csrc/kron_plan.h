@@ -161,6 +161,11 @@ struct alignas(16) FusedUnit {
 	int       rj;  // contraction of the first product (rows of X_j)
 	int       lj;  // leading dimension of A^T_k(i,j) (= l_j)
 	int       cw;  // columns of the unit (<= the configuration's unit width)
+	int       kind; // 0, or kSegXA / kSegXB: a term with an identity factor is one product,
+	                // cw wide along its contraction: Y_i += X_j(:, c0..) A^T(c0.., :) from
+	                // x_off (ld rj) and at_off (ld lj), or B(:, c0..) X_j(c0.., :) from b_off
+	                // (ld ldb) and x_off (ld rj)
+	int       pad;
 };
 
 // One CTA of the fused launch: part `part` of `nparts` of the output tile

@@ -1,4 +1,4 @@
-// Host emulation of the persistent FP64 H*x on sectors with identity blocks,
+// Host emulation of the persistent and fused FP64 H*x on sectors with identity blocks,
 // whose terms skip pass 1 (kSegXA, kSegXB in kron_plan.h), against H*x from the
 // caller's blocks with every identity multiplied out.
 // Usage: identity_schedule_check seed npatches max_size
@@ -134,6 +134,44 @@ int main(int argc, char** argv)
 			}
 		}
 
+	// the fused form's units (its tiles 32 rows high, 64 or 128 columns wide)
+	for (int bn : { 64, 128 }) {
+		build_fused_schedule(plan, 32, bn, 64, 8, 2, 1184);
+		const std::string verdict = validate_fused_schedule(plan, 32, bn, 8);
+		if (!verdict.empty())
+			return fail("fused validator: " + verdict);
+		std::vector<double> y(D, 0.0);
+		for (const FusedItem& it : plan.fitems) {
+			if (it.nparts == 0)
+				continue;
+			for (int n = it.n0; n < std::min(it.n0 + bn, it.N); ++n)
+				for (int m = it.m0; m < std::min(it.m0 + 32, it.M); ++m) {
+					double s = 0.0;
+					for (int u = it.u_begin; u < it.u_end; ++u) {
+						const FusedUnit& d = plan.funits[size_t(u)];
+						for (int c = 0; c < d.cw; ++c) {
+							double t = 0.0;
+							if (d.kind == kSegXA) {
+								t = x.at(size_t(d.x_off + m + (long long)c * d.rj));
+							} else if (d.kind == kSegXB) {
+								s += pack.at(size_t(d.b_off + m + (long long)c * d.ldb))
+								    * x.at(size_t(d.x_off + c + (long long)n * d.rj));
+								continue;
+							} else {
+								for (int k = 0; k < d.rj; ++k)
+									t += pack.at(size_t(d.b_off + m + (long long)k * d.ldb))
+									    * x.at(size_t(d.x_off + k + (long long)c * d.rj));
+							}
+							s += t * pack.at(size_t(d.at_off + c + (long long)n * d.lj));
+						}
+					}
+					y[size_t(it.y_off + m + (long long)n * it.M)] += s;
+				}
+		}
+		for (size_t q = 0; q < D; ++q)
+			if (!(std::fabs(y[q] - ref[q]) <= 1e-12 * scale))
+				return fail("fused H*x differs");
+	}
 	std::printf("ok %.2e %d\n", e64, idents);
 	return 0;
 }
