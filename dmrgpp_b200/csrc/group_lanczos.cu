@@ -654,14 +654,15 @@ k_g_pcg_sums(const double* __restrict__ res, const double* __restrict__ diag, co
 	}
 }
 
-// p = z + (rho_new / rho) p (p = z when first), rho_new = sums1 - a sums2,
-// a = sums0 / uw; every chunk of a sector computes the same rho_new, and its
-// sector's first chunk stores it in rho_next
+// p = z + (rho_new / rho) p (FIRST: p = z, neither p nor rho is read),
+// rho_new = sums1 - a sums2, a = sums0 / uw; every chunk of a sector computes
+// the same rho_new, and its sector's first chunk stores it in rho_next
+template <bool FIRST>
 __global__ void __launch_bounds__(kThreads)
 k_g_pcg_direction(double* __restrict__ p, const double* __restrict__ res, const double* __restrict__ diag,
                   const double* __restrict__ theta, const double* __restrict__ wv, const double* __restrict__ uw,
                   const double* __restrict__ sums, int nseg, const double* __restrict__ rho,
-                  double* __restrict__ rho_next, int first, const Chunk* __restrict__ chunks, int nch,
+                  double* __restrict__ rho_next, const Chunk* __restrict__ chunks, int nch,
                   const int* __restrict__ seg_chunk, const int* __restrict__ active)
 {
 	for (int ch = blockIdx.x; ch < nch; ch += gridDim.x) {
@@ -671,7 +672,7 @@ k_g_pcg_direction(double* __restrict__ p, const double* __restrict__ res, const 
 		const int    sg      = k.seg;
 		const double a       = uw[sg] > 0.0 ? sums[sg] / uw[sg] : 0.0;
 		const double rho_new = sums[nseg + sg] - a * sums[2 * nseg + sg];
-		const double beta    = first ? 0.0 : (rho[sg] > 0.0 ? rho_new / rho[sg] : 0.0);
+		const double beta    = FIRST ? 0.0 : (rho[sg] > 0.0 ? rho_new / rho[sg] : 0.0);
 		if (threadIdx.x == 0 && ch == seg_chunk[sg])
 			rho_next[sg] = rho_new;
 		const double th = theta[sg];
@@ -679,7 +680,7 @@ k_g_pcg_direction(double* __restrict__ p, const double* __restrict__ res, const 
 		for (int i = threadIdx.x; i < k.len; i += kThreads) {
 			const long long q = k.begin + i;
 			const double    z = res[q] / g_pcg_k(diag[q], th) - a * wv[q];
-			p[q]              = z + beta * p[q];
+			p[q]              = FIRST ? z : z + beta * p[q];
 		}
 	}
 }
@@ -1339,9 +1340,8 @@ extern "C" int dmrgpp_refine_lowest_group(dmrgpp_kron_handle h, double* psi, int
 			k_g_pcg_setup<<<grid, kThreads, 0, st>>>(psi, h->d_diag, theta, wv, w->chunks, nch, cg, w->rpart);
 			k_g_finish<<<S, kThreads, 0, st>>>(w->rpart, w->seg_chunk, cg, uw, 0);
 			pcg_sums();
-			// first = 1: rho is not read, the other half of its double buffer stands in
-			k_g_pcg_direction<<<grid, kThreads, 0, st>>>(pv, res, h->d_diag, theta, wv, uw, sums, S, rho[1],
-			                                             rho[0], 1, w->chunks, nch, w->seg_chunk, cg);
+			k_g_pcg_direction<true><<<grid, kThreads, 0, st>>>(pv, res, h->d_diag, theta, wv, uw, sums, S, nullptr,
+			                                                   rho[0], w->chunks, nch, w->seg_chunk, cg);
 		}
 		int cur = 0, inner = 0;
 		while (inner < inner_iterations) {
@@ -1362,9 +1362,9 @@ extern "C" int dmrgpp_refine_lowest_group(dmrgpp_kron_handle h, double* psi, int
 				                                         b0, inner_tolerance, jac ? h->d_diag : nullptr, theta, psi,
 				                                         wv, sums, w->chunks, nch, S, cg, w->rpart, sg);
 				if (jac) {
-					k_g_pcg_direction<<<grid, kThreads, 0, st>>>(pv, res, h->d_diag, theta, wv, uw, sums, S,
-					                                             rho[cur], rho[cur ^ 1], 0, w->chunks, nch,
-					                                             w->seg_chunk, cg);
+					k_g_pcg_direction<false><<<grid, kThreads, 0, st>>>(pv, res, h->d_diag, theta, wv, uw, sums, S,
+					                                                    rho[cur], rho[cur ^ 1], w->chunks, nch,
+					                                                    w->seg_chunk, cg);
 				} else {
 					k_g_cg_direction<<<grid, kThreads, 0, st>>>(pv, res, rr[cur ^ 1], rr[cur], w->chunks, nch,
 					                                            cg);

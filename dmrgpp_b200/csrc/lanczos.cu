@@ -1564,26 +1564,27 @@ k_pcg_update(double* __restrict__ t, double* __restrict__ res, const double* __r
 }
 
 // z = K^-1 res - a wv with a = sums[0] / *uw; rho_new = sums[1] - a sums[2];
-// p = z + (rho_new / *rho) p (p = z when first); *rho_next = rho_new.
-// Skipped once the iteration is frozen.
+// p = z + (rho_new / *rho) p; *rho_next = rho_new.  FIRST: p = z, and neither p
+// nor *rho is read: p is scratch that nothing has written yet, and a NaN there
+// would survive a factor of 0.  Skipped once the iteration is frozen.
+template <bool FIRST>
 __global__ void __launch_bounds__(kThreads)
 k_pcg_direction(double* __restrict__ p, const double* __restrict__ res, const double* __restrict__ diag,
                 double theta, double floor_, const double* __restrict__ wv, const double* uw,
-                const double* sums, const double* rho, double* rho_next, const double* broken, int first,
-                size_t n)
+                const double* sums, const double* rho, double* rho_next, const double* broken, size_t n)
 {
 	if (*broken != 0.0)
 		return;
 	const double a       = *uw > 0.0 ? sums[0] / *uw : 0.0;
 	const double rho_new = sums[1] - a * sums[2];
-	const double beta    = first ? 0.0 : (*rho > 0.0 ? rho_new / *rho : 0.0);
+	const double beta    = FIRST ? 0.0 : (*rho > 0.0 ? rho_new / *rho : 0.0);
 	if (blockIdx.x == 0 && threadIdx.x == 0)
 		*rho_next = rho_new;
 #pragma unroll 4
 	for (size_t i = blockIdx.x * size_t(kThreads) + threadIdx.x; i < n;
 	     i += size_t(gridDim.x) * kThreads) {
 		const double z = res[i] / pcg_k(diag[i], theta, floor_) - a * wv[i];
-		p[i]           = z + beta * p[i];
+		p[i]           = FIRST ? z : z + beta * p[i];
 	}
 }
 
@@ -1618,8 +1619,8 @@ int pcg_correction(dmrgpp_kron_handle h, const double* u, double theta, const do
 	};
 	k_pcg_setup<<<nb, kThreads, 0, st>>>(u, h->d_diag, theta, floor_, wv, D, sc + 5, w->partial, w->ctr + 8);
 	k_pcg_sums<<<nb, kThreads, 0, st>>>(res, h->d_diag, theta, floor_, u, wv, D, sc + 6, w->partial, w->ctr + 9);
-	k_pcg_direction<<<nb, kThreads, 0, st>>>(p, res, h->d_diag, theta, floor_, wv, sc + 5, sc + 6, sc + 10,
-	                                         sc + 10, sc + 4, 1, D);
+	k_pcg_direction<true><<<nb, kThreads, 0, st>>>(p, res, h->d_diag, theta, floor_, wv, sc + 5, sc + 6, nullptr,
+	                                               sc + 10, sc + 4, D);
 	double host[4] = { 0, 0, 0, 0 };
 	if (!read(sc + 9, 1, host))
 		return handle_fail(h, DMRGPP_CUDA_ERROR, "correction solve");
@@ -1638,8 +1639,8 @@ int pcg_correction(dmrgpp_kron_handle h, const double* u, double theta, const do
 			k_cg_curvature<<<nb, kThreads, 0, st>>>(Aq, p, u, theta, sc + 0, D, sc + 1, w->partial, w->ctr + 7);
 			k_pcg_update<<<nb, kThreads, 0, st>>>(t, res, p, Aq, sc + 10 + cur, sc + 1, sc + 4, h->d_diag,
 			                                      theta, floor_, u, wv, D, sc + 6, w->partial, w->ctr + 9);
-			k_pcg_direction<<<nb, kThreads, 0, st>>>(p, res, h->d_diag, theta, floor_, wv, sc + 5, sc + 6,
-			                                         sc + 10 + cur, sc + 11 - cur, sc + 4, 0, D);
+			k_pcg_direction<false><<<nb, kThreads, 0, st>>>(p, res, h->d_diag, theta, floor_, wv, sc + 5, sc + 6,
+			                                                sc + 10 + cur, sc + 11 - cur, sc + 4, D);
 			cur ^= 1;
 		}
 		if ((e = cudaGetLastError()))
