@@ -117,6 +117,7 @@ k_tridiag(double* __restrict__ rho, double* __restrict__ work, const TridiagJob*
 	__shared__ double                      red[kTriThreads / 32];
 	__shared__ double                      amax_of[kTriCluster];
 	cg::cluster_group                      cluster = cg::this_cluster();
+	cluster.barrier_arrive(); // this CTA runs: its shared memory may be written to (waited for below)
 	const int                              rank    = int(cluster.block_rank());
 	const int                              tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const TridiagJob                       jb = jobs[blockIdx.x / kTriCluster];
@@ -147,6 +148,7 @@ k_tridiag(double* __restrict__ rho, double* __restrict__ work, const TridiagJob*
 	if (lane == 0)
 		red[warp] = amax;
 	__syncthreads();
+	cluster.barrier_wait(); // every CTA of the cluster has started: the stores below go to their shared memory
 	if (tid < kTriCluster) {
 		double m = 0.0;
 		for (int w = 0; w < kTriThreads / 32; ++w)

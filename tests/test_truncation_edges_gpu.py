@@ -44,6 +44,16 @@ def test_group_sizes(cuda_lib, cuda_device, sizes):
     _check(sizes, rights, psi / np.linalg.norm(psi), max(1, sum(sizes) // 3))
 
 
+def test_many_small_groups(cuda_lib, cuda_device):
+    """More clusters than run at once, most of their CTAs without a column:
+    a CTA reaches its first store to the others' shared memory at once."""
+    rng = np.random.default_rng(9)
+    sizes = [int(n) for n in rng.integers(1, 10, 900)]
+    rights = [int(n) for n in rng.integers(1, 12, 900)]
+    psi = np.concatenate([rng.standard_normal(n * r) for n, r in zip(sizes, rights)])
+    _check(sizes, rights, psi / np.linalg.norm(psi), sum(sizes) // 2)
+
+
 @pytest.mark.parametrize("weight", [1e-14, 1e-60, 1e60])
 def test_weights_outside_the_reductions_range(cuda_lib, cuda_device, weight):
     rng = np.random.default_rng(4)
