@@ -1101,6 +1101,13 @@ int dmrgpp_kron_apply(dmrgpp_kron_handle h, const double* x, double* y, int on_d
 	if (!on_device
 	    && (e = cudaMemcpyAsync(h->d_x, x, dim * sizeof(double), cudaMemcpyHostToDevice, h->stream)))
 		return cuda_fail(h, e, "copy x to device");
+	// y over x: the FP64 forms read X (terms with an identity factor, the fused
+	// form) while other CTAs of the launch write Y; the TF32x3 form splits X first
+	if (on_device && h->precision == DMRGPP_FP64 && dmrgpp::vectors_overlap(x, y, dim)) {
+		if ((e = cudaMemcpyAsync(h->d_x, x, dim * sizeof(double), cudaMemcpyDeviceToDevice, h->stream)))
+			return cuda_fail(h, e, "copy x");
+		X = h->d_x;
+	}
 
 	if (int rc = dmrgpp::kron_apply_device(h, X, Y))
 		return rc;

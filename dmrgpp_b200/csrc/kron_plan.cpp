@@ -95,6 +95,13 @@ void order_tiles(std::vector<GemmTile>& tiles, const std::vector<GemmSeg>& segs)
 // 0: B_k(i,j) X_j (A is the identity), 1: X_j A^T (B is), 2: both products
 static int term_kind(int ident) { return ident & kIdentB ? 1 : ident & kIdentA ? 0 : 2; }
 
+void multiply_out_identities(KronPlan& plan)
+{
+	plan.ident.assign(plan.triples.size(), 0);
+	plan.M1 = plan.M;
+	build_tile_lists(plan, plan.bm, plan.bn);
+}
+
 void build_tile_lists(KronPlan& plan, int bm, int bn)
 {
 	const size_t np = plan.np;

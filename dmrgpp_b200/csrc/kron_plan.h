@@ -23,6 +23,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstdint>
 #include <thread>
 #include <cstddef>
 #include <cstdint>
@@ -253,6 +254,13 @@ struct MixedPlan {
 	long long              split_slots   = 0; // partial tiles of their parts
 };
 
+// Whether [x, x + n) and [y, y + n) share an element.
+inline bool vectors_overlap(const double* x, const double* y, size_t n)
+{
+	const uintptr_t a = reinterpret_cast<uintptr_t>(x), b = reinterpret_cast<uintptr_t>(y);
+	return (a < b ? b - a : a - b) < n * sizeof(double);
+}
+
 struct KronPlan {
 	size_t np = 0, nop = 0;
 	std::vector<long long> l, r;        // patch sizes
@@ -420,6 +428,11 @@ void split_tf32(double v, float* hi, float* lo);
 // (Re)builds the two-launch tile lists seg1/tile1/seg2/tile2 of a planned
 // sector for bm x bn output tiles.
 void build_tile_lists(KronPlan& plan, int bm, int bn);
+
+// Gives a planned sector's identity factors up as such: every term is two
+// products again, so that pass 1 is the only reader of X (the tile lists are
+// rebuilt; the packed operators stay as they are).
+void multiply_out_identities(KronPlan& plan);
 
 // Reorders the tiles of one tensor-core pass into per-CTA runs: CTA b of the
 // persistent launch processes tiles [starts[b], starts[b+1]).  Tiles go,

@@ -105,6 +105,10 @@ int dmrgpp_kron_apply_noalloc(const dmrgpp_kron_desc* d, const double* x, double
                                               &pack);
 	if (!msg.empty())
 		return noalloc_fail(DMRGPP_INVALID_ARG, msg);
+	// y over x: pass 2 must not read X while it writes Y (one buffer each, no
+	// third one to copy x to)
+	if (dmrgpp::vectors_overlap(x, y, size_t(plan.dim())))
+		dmrgpp::multiply_out_identities(plan);
 
 	// scratch layout: [packed operators | BX | segments and tiles]
 	const size_t ops_bytes  = size_t(plan.op_elems) * sizeof(double);

@@ -148,7 +148,8 @@ int dmrgpp_kron_destroy(dmrgpp_kron_handle h);
  * apply_Htarget_sparse_not_ready.cpp:14-478): y = H x (overwrite) in patch
  * order.  on_device = 0: x and y are host pointers (copied in and out on the
  * handle's stream; the call returns when y is written).  on_device = 1: x
- * and y are device pointers; the call only enqueues work on the stream. */
+ * and y are device pointers; the call only enqueues work on the stream.  x
+ * and y may be the same buffer or overlap. */
 int dmrgpp_kron_apply(dmrgpp_kron_handle h, const double* x, double* y, int on_device);
 
 /* Switches the arithmetic of later applies (and of the eigensolvers) between
@@ -255,7 +256,8 @@ int dmrgpp_kron_plan_info_get(const dmrgpp_kron_desc* desc, dmrgpp_kron_plan_inf
  * code running while another component owns all device memory through its
  * own allocator, or a runtime that forbids allocation after start-up).
  * desc is read as by dmrgpp_kron_create (host tables, FP64 only); x and y
- * are device pointers of the sector dimension; the work is enqueued on
+ * are device pointers of the sector dimension, which may be the same or
+ * overlap (every term then is two products); the work is enqueued on
  * desc->stream and the call returns without waiting for it.
  * All scratch (packed operators, the pass-1 buffer, launch lists) lives in
  * one file-scope device array of DMRGPP_NOALLOC_SCRATCH_BYTES that every GPU
