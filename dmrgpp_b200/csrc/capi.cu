@@ -136,42 +136,6 @@ void pick_tile(const dmrgpp_kron_desc* d, int& bm, int& bn)
 	pick_tile_sizes(d->npatches, d->left_patch_size, d->right_patch_size, bm, bn);
 }
 
-// The FP64 configuration of a new handle (the tuner replaces it by the fastest
-// on the sector itself).  Where the lines lie, from sweeps of spin links,
-// Hubbard chains and ladders and sector groups on a B200 (us per H*x):
-// * few patches, each within one fused column tile: the fused form has no
-//   dependent second pass (5 to 21 patches: 8.5 against 11.5 with two passes,
-//   12.4 against 16.5, microbench sector 27.6 against 34.8); with many small
-//   patches its units are too short (145 patches: 33 against 32), and above
-//   4e8 flops the heaviest part sets its end (6e8: 126 against 72);
-// * small work: 32 x 32 tiles with k-chunks of 32, half as many steps in the
-//   latency-bound chains (chain of 4000 states 49.3 against 56.1 with chunks
-//   of 16); from 6e8 flops shorter chunks waste less of ragged patches
-//   (batch of 8 sectors 66.5 against 70.0) unless patches are wide (ladder of
-//   10000 states, patches to 332: 445 against 460);
-// * 64 x 64 tiles only where the sector fills the SMs several times over with
-//   them: 1396 against 1449 at 3.6e10 flops, but 740 against 700 at 1.6e10
-//   and 2 to 4 times slower below 1e9.
-void default_config(const dmrgpp::KronPlan& P, int* cfg, int* ipc)
-{
-	long long widest = 0, max_l = 0;
-	for (size_t p = 0; p < P.np; ++p) {
-		max_l  = std::max(max_l, P.l[p]);
-		widest = std::max({ widest, P.l[p], P.r[p] });
-	}
-	*ipc = 2;
-	if (P.np <= 40 && max_l <= dmrgpp::fused_shape(0).bn && P.f_alg < 4e8) {
-		*cfg = dmrgpp::kNumTileCfgs;
-		*ipc = 1;
-	} else if (P.f_alg >= 2.5e10) {
-		*cfg = 2;
-	} else if (P.f_alg >= 6e8 && widest < 320) {
-		*cfg = 0;
-	} else {
-		*cfg = 1;
-	}
-}
-
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no
 // direct libcuda dependency)
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
@@ -660,9 +624,14 @@ int finish_create(dmrgpp_kron_handle h, int device, void* stream, Clock::time_po
 
 	if ((e = dmrgpp::error_word_alloc(&h->err_host, &h->err_dev)))
 		return bail(e, "error word");
-	int cfg = 0, ipc = 0;
-	default_config(P, &cfg, &ipc);
-	if (int rc = dmrgpp::configure_schedule(h, cfg, ipc)) {
+	dmrgpp::DefaultConfig dc = dmrgpp::default_config(P, dmrgpp::fused_shape(0).bn);
+	int                   clusters = 0;
+	if (dc.fused && (dmrgpp::fused_init(0, &clusters) != cudaSuccess || clusters < 1)) {
+		// no cluster of the fused form fits (a share of the SMs, say): two passes
+		cudaGetLastError();
+		dc = dmrgpp::default_config(P, 0);
+	}
+	if (int rc = dmrgpp::configure_schedule(h, dc.fused ? dmrgpp::kNumTileCfgs : dc.cfg, dc.items_per_cta)) {
 		const std::string why = h->err;
 		release(h);
 		delete h;

@@ -490,6 +490,36 @@ bool validation_requested()
 	return on;
 }
 
+// The FP64 configuration of a new handle (the tuner replaces it by the fastest
+// on the sector itself).  Where the lines lie, from sweeps of spin links,
+// Hubbard chains and ladders and sector groups on a B200 (us per H*x):
+// * few patches, each within one fused column tile: the fused form has no
+//   dependent second pass (5 to 21 patches: 8.5 against 11.5 with two passes,
+//   12.4 against 16.5, microbench sector 27.6 against 34.8); with many small
+//   patches its units are too short (145 patches: 33 against 32), and above
+//   4e8 flops the heaviest part sets its end (6e8: 126 against 72);
+// * small work: 32 x 32 tiles with k-chunks of 32, half as many steps in the
+//   latency-bound chains (chain of 4000 states 49.3 against 56.1 with chunks
+//   of 16); from 6e8 flops shorter chunks waste less of ragged patches
+//   (batch of 8 sectors 66.5 against 70.0) unless patches are wide (ladder of
+//   10000 states, patches to 332: 445 against 460);
+// * 64 x 64 tiles only where the sector fills the SMs several times over with
+//   them: 1396 against 1449 at 3.6e10 flops, but 740 against 700 at 1.6e10
+//   and 2 to 4 times slower below 1e9.
+DefaultConfig default_config(const KronPlan& plan, long long fused_bn)
+{
+	long long widest = 0, max_l = 0;
+	for (size_t p = 0; p < plan.np; ++p) {
+		max_l  = std::max(max_l, plan.l[p]);
+		widest = std::max({ widest, plan.l[p], plan.r[p] });
+	}
+	if (plan.np <= 40 && max_l <= fused_bn && plan.f_alg < 4e8)
+		return { true, 0, 1 };
+	if (plan.f_alg >= 2.5e10)
+		return { false, 2, 2 };
+	return { false, plan.f_alg >= 6e8 && widest < 320 ? 0 : 1, 2 };
+}
+
 std::string validate_persistent_schedule(const KronPlan& plan, int tile)
 {
 	const long long dim = plan.dim(), ops = plan.op_elems, bx = plan.bx_elems;
