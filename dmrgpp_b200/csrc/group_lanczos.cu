@@ -1307,8 +1307,13 @@ extern "C" int dmrgpp_refine_lowest_group(dmrgpp_kron_handle h, double* psi, int
 			// a sector whose residual has not halved over two outer steps
 			// is failing (its start lies above the first excitation, where
 			// the projected correction equation is indefinite): it stops
-			// here, unconverged, instead of holding the lockstep launches
-			if (rn_h[q] < 0.5 * best[size_t(q)]) {
+			// here, unconverged, instead of holding the lockstep launches;
+			// one that is not finite never will be
+			if (!std::isfinite(rn_h[q]) || !std::isfinite(th_h[q])) {
+				act[size_t(q)] = 0;
+				--n_active;
+				changed = true;
+			} else if (rn_h[q] < 0.5 * best[size_t(q)]) {
 				best[size_t(q)]  = rn_h[q];
 				stall[size_t(q)] = 0;
 			} else if (++stall[size_t(q)] >= 2) {

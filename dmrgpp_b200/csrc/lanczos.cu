@@ -1594,6 +1594,17 @@ k_pcg_direction(double* __restrict__ p, const double* __restrict__ res, const do
 namespace dmrgpp {
 namespace {
 
+// A correction solve whose |res|^2 is not finite (not a number in r, u or H*x,
+// or an overflow): t is worth nothing, and the caller is told so.
+int correction_not_finite(dmrgpp_kron_handle h, int it, int* iterations, double* rel_residual)
+{
+	if (iterations)
+		*iterations = it;
+	if (rel_residual)
+		*rel_residual = std::numeric_limits<double>::quiet_NaN();
+	return handle_fail(h, DMRGPP_NOT_CONVERGED, "correction solve: the residual is not finite");
+}
+
 // The correction equation by conjugate gradients with the projected
 // diagonal preconditioner (see k_pcg_setup); res (= -P r on entry, as the
 // caller set it) and the Davidson buffers as in dmrgpp_correction_solve;
@@ -1624,6 +1635,8 @@ int pcg_correction(dmrgpp_kron_handle h, const double* u, double theta, const do
 	double host[4] = { 0, 0, 0, 0 };
 	if (!read(sc + 9, 1, host))
 		return handle_fail(h, DMRGPP_CUDA_ERROR, "correction solve");
+	if (!std::isfinite(host[0]))
+		return correction_not_finite(h, 0, iterations, rel_residual);
 	const double b0  = std::sqrt(host[0]);
 	double       rrh = host[0];
 	int          it  = 0;
@@ -1652,6 +1665,8 @@ int pcg_correction(dmrgpp_kron_handle h, const double* u, double theta, const do
 		if (four[0] != 0.0)
 			break; // the projected operator was not positive definite
 	}
+	if (!std::isfinite(rrh))
+		return correction_not_finite(h, it, iterations, rel_residual);
 	if (iterations)
 		*iterations = it;
 	if (rel_residual)
@@ -1732,6 +1747,8 @@ int dmrgpp_correction_solve(dmrgpp_kron_handle h, const double* u, double theta,
 	double host[4] = { 0, 0, 0, 0 };
 	if (!read(sc + 2, 1, host))
 		return handle_fail(h, DMRGPP_CUDA_ERROR, "correction solve");
+	if (!std::isfinite(host[0]))
+		return correction_not_finite(h, 0, iterations, rel_residual);
 	const double b0  = std::sqrt(host[0]);
 	double       rrh = host[0];
 	int          it  = 0;
@@ -1757,6 +1774,8 @@ int dmrgpp_correction_solve(dmrgpp_kron_handle h, const double* u, double theta,
 		if (host[2] != 0.0)
 			break; // the projected operator was not positive definite
 	}
+	if (!std::isfinite(rrh))
+		return correction_not_finite(h, it, iterations, rel_residual);
 	if (iterations)
 		*iterations = it;
 	if (rel_residual)
@@ -1845,7 +1864,7 @@ int dmrgpp_refine_lowest(dmrgpp_kron_handle h, double* psi, int max_outer, doubl
 			s.converged = 1;
 			break;
 		}
-		if (outer == max_outer)
+		if (outer == max_outer || !std::isfinite(theta) || !std::isfinite(rnorm))
 			break;
 		// a residual that has not halved over two outer steps means a failing
 		// refinement (start above the first excitation): stop, unconverged
@@ -1857,8 +1876,12 @@ int dmrgpp_refine_lowest(dmrgpp_kron_handle h, double* psi, int max_outer, doubl
 		}
 		int    its = 0;
 		double rel = 0.0;
-		if ((rc = dmrgpp_correction_solve(h, psi, theta, r, t, inner_iterations, inner_tolerance, &its,
-		                                  &rel)))
+		rc = dmrgpp_correction_solve(h, psi, theta, r, t, inner_iterations, inner_tolerance, &its, &rel);
+		if (rc == DMRGPP_NOT_CONVERGED) { // not finite: psi stays as it is
+			rc = DMRGPP_OK;
+			break;
+		}
+		if (rc)
 			break;
 		s.inner_matvecs += size_t(its);
 		k_axpy<<<nb, kThreads, 0, st>>>(1.0, t, psi, D);

@@ -410,7 +410,9 @@ int dmrgpp_davidson_lowest(dmrgpp_kron_handle h, const dmrgpp_davidson_params* p
 /* Exact correction for training the learned preconditioner: solves
  * (I - u u^T)(H - theta)(I - u u^T) t = -r, t orthogonal to u, by conjugate
  * gradients in FP64 on the device (u unit norm, r orthogonal to u, theta
- * below the second eigenvalue).  All vectors are device pointers. */
+ * below the second eigenvalue).  All vectors are device pointers.  Returns
+ * DMRGPP_NOT_CONVERGED when the residual is not finite (NaN in the inputs, or
+ * an overflow). */
 int dmrgpp_correction_solve(dmrgpp_kron_handle h, const double* u, double theta, const double* r,
                             double* t, int max_iterations, double rel_tolerance, int* iterations,
                             double* rel_residual);
@@ -433,7 +435,9 @@ int dmrgpp_set_correction_preconditioner(dmrgpp_kron_handle h, int preconditione
  * (I - psi psi^T)(H - theta)(I - psi psi^T) t = -r by conjugate gradients
  * with the handle's current (mixed) matvecs (inner_iterations,
  * inner_tolerance) and sets psi <- (psi + t) / |psi + t|.  energy = final
- * FP64 Rayleigh quotient.  No counterpart in the reference. */
+ * FP64 Rayleigh quotient.  A correction or a Rayleigh quotient that is not
+ * finite ends it with DMRGPP_NOT_CONVERGED, psi as the last good step left it.
+ * No counterpart in the reference. */
 typedef struct {
 	size_t outer_iterations;
 	size_t inner_matvecs; /* matvecs of the correction solves (handle precision) */
