@@ -10,7 +10,8 @@
 // transformation is U.  Here rho_g = M_g M_g^T is formed directly as a sum of
 // X_p^T X_p (system side) or X_p X_p^T (environment side) by one grouped DGEMM
 // launch on the FP64 tensor pipe and reduced to tridiagonal form there, one
-// cluster of CTAs per group, their eigenvalues found by bisection; the host
+// cluster of CTAs per group, their eigenvalues found by bisection (groups above
+// kTriMaxN states go to the host cores meanwhile: tridiag.cpp); the host
 // ranks the states (computeKeptStates) and forms the kept eigenvectors of the
 // tridiagonals by inverse iteration on all cores (tridiag.cpp), and the device
 // applies the Householder reflectors to them.
@@ -71,6 +72,7 @@ namespace cg = cooperative_groups;
 // One group of the tridiagonal reduction.
 struct TridiagJob {
 	long long m_off; // rho_g (n x n)
+	long long w_off; // its working copy
 	long long e_off; // its place in the per-state arrays
 	int       n;
 	int       group;
@@ -123,7 +125,7 @@ k_tridiag(double* __restrict__ rho, double* __restrict__ work, const TridiagJob*
 	const TridiagJob                       jb = jobs[blockIdx.x / kTriCluster];
 	const int                              n  = jb.n;
 	double*                                R  = rho + jb.m_off;
-	double*                                A  = work + jb.m_off;
+	double*                                A  = work + jb.w_off;
 	d += jb.e_off;
 	off += jb.e_off;
 	beta += jb.e_off;
@@ -462,6 +464,27 @@ k_back_transform(const double* __restrict__ z, double* __restrict__ v, const dou
 	}
 }
 
+// Largest group that k_tridiag takes on this device, 0 where no cluster of it
+// fits (a restricted share of the SMs, say).
+cudaError_t tridiag_limit(size_t* n)
+{
+	const size_t smem = 5 * size_t(kTriMaxN) * sizeof(double);
+	cudaError_t  e = cudaFuncSetAttribute(k_tridiag, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+	if (e)
+		return e;
+	cudaLaunchConfig_t cfg {};
+	cfg.gridDim          = dim3(kTriCluster, 1, 1);
+	cfg.blockDim         = dim3(kTriThreads, 1, 1);
+	cfg.dynamicSmemBytes = smem;
+	int clusters         = 0;
+	if (cudaOccupancyMaxActiveClusters(&clusters, k_tridiag, &cfg) != cudaSuccess) {
+		cudaGetLastError();
+		clusters = 0;
+	}
+	*n = clusters > 0 ? size_t(kTriMaxN) : 0;
+	return cudaSuccess;
+}
+
 // Truncation.h:476-512 (eigs ascending; tolerance < 0 keeps keptStates)
 size_t compute_kept(size_t kept_states, double tolerance, size_t m_min, const std::vector<double>& eigs)
 {
@@ -714,11 +737,35 @@ extern "C" int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, d
 	auto                        not_converged = [&](size_t g) {
         return fail(DMRGPP_NOT_CONVERGED, "eigensolver of group " + std::to_string(g) + " did not converge");
 	};
-	// reduction and eigenvalues on the device; groups whose vectors do not fit
-	// its shared memory make the host cores do it
-	const bool  on_device = nmax <= size_t(kTriMaxN);
-	double *    work = nullptr, *tri = nullptr; // tri: d, off, eigenvalues, beta (N each)
-	void*       d_tj = nullptr;
+	// reduction and eigenvalues of every group on the device, except of those
+	// whose vectors do not fit its shared memory: the host cores take these
+	// meanwhile
+	size_t limit = 0;
+	if ((e = tridiag_limit(&limit)))
+		return cuda_fail(e, "tridiagonal kernel attributes");
+	std::vector<size_t>     hg; // groups of the host, and their places in its buffers
+	std::vector<long long>  hoff(1, 0);
+	std::vector<TridiagJob> tj;
+	std::vector<BisectJob>  bj;
+	long long               work_elems = 0;
+	int                     vec        = 1; // largest group of the device
+	for (size_t g : by_size) {
+		const int n = int(d->group_size[g]);
+		if (n == 0)
+			continue;
+		if (size_t(n) > limit) {
+			hg.push_back(g);
+			hoff.push_back(hoff.back() + (long long)n * n);
+			continue;
+		}
+		tj.push_back({ goff[g], work_elems, eoff[g], n, int(g) });
+		work_elems += (long long)n * n;
+		vec = std::max(vec, n);
+		for (int k0 = 0; k0 < n; k0 += kBisThreads / 8)
+			bj.push_back({ eoff[g], n, k0 });
+	}
+	double *work = nullptr, *tri = nullptr; // tri: d, off, eigenvalues, beta (N each)
+	void*   d_tj = nullptr;
 	struct FreeT {
 		double **a, **b;
 		void**   c;
@@ -729,96 +776,93 @@ extern "C" int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, d
 			dev_free(*c);
 		}
 	} freet { &work, &tri, &d_tj };
-	Clock::time_point tp;
-	if (on_device) {
-		if ((e = cudaGetLastError()))
+	// the lists and the groups' shifts in one allocation
+	const size_t tjb = tj.size() * sizeof(TridiagJob), bjb = bj.size() * sizeof(BisectJob);
+	std::vector<unsigned char> lists(tjb + bjb);
+	std::copy_n(reinterpret_cast<const unsigned char*>(tj.data()), tjb, lists.data());
+	std::copy_n(reinterpret_cast<const unsigned char*>(bj.data()), bjb, lists.data() + tjb);
+	const size_t N1    = std::max<size_t>(N, 1);
+	double*      h_tri = pinned<double>(0, 3 * N1 + (ng + 1) / 2 + 1);
+	double*      h_rho = pinned<double>(1, size_t(hoff.back()));
+	if (!h_tri || !h_rho)
+		return fail(DMRGPP_OOM, "page-locked host buffers for the density matrices");
+	int*         h_shift  = reinterpret_cast<int*>(h_tri + 3 * N1);
+	const size_t tri_smem = 5 * size_t(vec) * sizeof(double), bis_smem = 2 * size_t(vec) * sizeof(double);
+	if ((e = cudaGetLastError()) || (e = dev_malloc(&work, size_t(std::max(work_elems, 1LL)) * sizeof(double)))
+	    || (e = dev_malloc(&tri, 4 * N1 * sizeof(double)))
+	    || (e = dev_malloc(&d_tj, lists.size() + ng * sizeof(int) + 16)))
+		return cuda_fail(e, "tridiagonal allocation");
+	unsigned char* lp      = static_cast<unsigned char*>(d_tj);
+	int*           d_shift = reinterpret_cast<int*>(lp + lists.size());
+	if (!lists.empty() && (e = cudaMemcpyAsync(lp, lists.data(), lists.size(), cudaMemcpyHostToDevice, st)))
+		return cuda_fail(e, "tridiagonal set-up");
+	struct Event {
+		cudaEvent_t v = nullptr;
+		~Event()
+		{
+			if (v)
+				cudaEventDestroy(v);
+		}
+	} copied; // the host's density matrices are there
+	if (!hg.empty()) {
+		for (size_t q = 0; q < hg.size(); ++q)
+			if ((e = cudaMemcpyAsync(h_rho + hoff[q], rho + goff[hg[q]], size_t(hoff[q + 1] - hoff[q]) * sizeof(double),
+			                         cudaMemcpyDeviceToHost, st)))
+				return cuda_fail(e, "density matrices");
+		if ((e = cudaEventCreateWithFlags(&copied.v, cudaEventDisableTiming)) || (e = cudaEventRecord(copied.v, st)))
 			return cuda_fail(e, "density matrices");
-		std::vector<TridiagJob> tj;
-		std::vector<BisectJob>  bj;
-		for (size_t g : by_size) {
-			const int n = int(d->group_size[g]);
-			if (n == 0)
-				continue;
-			tj.push_back({ goff[g], eoff[g], n, int(g) });
-			for (int k0 = 0; k0 < n; k0 += kBisThreads / 8)
-				bj.push_back({ eoff[g], n, k0 });
+	}
+	double *dd = tri, *doff = tri + N1, *dw = tri + 2 * N1, *dbeta = tri + 3 * N1;
+	if (!tj.empty()) {
+		k_tridiag<<<unsigned(tj.size() * kTriCluster), kTriThreads, tri_smem, st>>>(
+		    rho, work, reinterpret_cast<const TridiagJob*>(lp), dd, doff, dbeta, d_shift, vec);
+		k_bisect<<<unsigned(bj.size()), kBisThreads, bis_smem, st>>>(
+		    dd, doff, dw, reinterpret_cast<const BisectJob*>(lp + tjb));
+	}
+	if ((e = cudaGetLastError())
+	    || (e = cudaMemcpyAsync(h_tri, tri, 3 * N1 * sizeof(double), cudaMemcpyDeviceToHost, st))
+	    || (e = cudaMemcpyAsync(h_shift, d_shift, ng * sizeof(int), cudaMemcpyDeviceToHost, st)))
+		return cuda_fail(e, "tridiagonal reduction");
+	g_trunc_times[DMRGPP_TRUNC_RHO] = seconds_since(t_start);
+	auto tp                         = Clock::now();
+	ge.assign(ng, GroupReduction {});
+	if (!hg.empty()) {
+		if ((e = cudaEventSynchronize(copied.v)))
+			return cuda_fail(e, "density matrices");
+		std::vector<GroupReduction> red;
+		std::vector<size_t>         hn;
+		std::vector<double*>        ga, gw;
+		for (size_t q = 0; q < hg.size(); ++q) {
+			hn.push_back(d->group_size[hg[q]]);
+			ga.push_back(h_rho + hoff[q]);
+			gw.push_back(eigenvalues + eoff[hg[q]]);
 		}
-		// the lists and the groups' shifts in one allocation
-		const size_t tjb = tj.size() * sizeof(TridiagJob), bjb = bj.size() * sizeof(BisectJob);
-		std::vector<unsigned char> lists(tjb + bjb);
-		std::copy_n(reinterpret_cast<const unsigned char*>(tj.data()), tjb, lists.data());
-		std::copy_n(reinterpret_cast<const unsigned char*>(bj.data()), bjb, lists.data() + tjb);
-		const size_t N1 = std::max<size_t>(N, 1);
-		double*      h_tri = pinned<double>(0, 3 * N1 + (ng + 1) / 2 + 1);
-		if (!h_tri)
-			return fail(DMRGPP_OOM, "page-locked host buffer for the tridiagonals");
-		int*       h_shift = reinterpret_cast<int*>(h_tri + 3 * N1);
-		const int  vec     = int(std::max<size_t>(nmax, 1));
-		const size_t tri_smem = 5 * size_t(vec) * sizeof(double), bis_smem = 2 * size_t(vec) * sizeof(double);
-		if ((e = dev_malloc(&work, rho_elems * sizeof(double))) || (e = dev_malloc(&tri, 4 * N1 * sizeof(double)))
-		    || (e = dev_malloc(&d_tj, lists.size() + ng * sizeof(int) + 16))
-		    || (e = cudaFuncSetAttribute(k_tridiag, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                                 int(5 * size_t(kTriMaxN) * sizeof(double)))))
-			return cuda_fail(e, "tridiagonal allocation");
-		unsigned char* lp      = static_cast<unsigned char*>(d_tj);
-		int*           d_shift = reinterpret_cast<int*>(lp + lists.size());
-		if (!lists.empty() && (e = cudaMemcpyAsync(lp, lists.data(), lists.size(), cudaMemcpyHostToDevice, st)))
-			return cuda_fail(e, "tridiagonal set-up");
-		double *dd = tri, *doff = tri + N1, *dw = tri + 2 * N1, *dbeta = tri + 3 * N1;
-		if (!tj.empty()) {
-			k_tridiag<<<unsigned(tj.size() * kTriCluster), kTriThreads, tri_smem, st>>>(
-			    rho, work, reinterpret_cast<const TridiagJob*>(lp), dd, doff, dbeta, d_shift, vec);
-			k_bisect<<<unsigned(bj.size()), kBisThreads, bis_smem, st>>>(
-			    dd, doff, dw, reinterpret_cast<const BisectJob*>(lp + tjb));
-		}
-		if ((e = cudaGetLastError())
-		    || (e = cudaMemcpyAsync(h_tri, tri, 3 * N1 * sizeof(double), cudaMemcpyDeviceToHost, st))
-		    || (e = cudaMemcpyAsync(h_shift, d_shift, ng * sizeof(int), cudaMemcpyDeviceToHost, st)))
-			return cuda_fail(e, "tridiagonal reduction");
-		g_trunc_times[DMRGPP_TRUNC_RHO] = seconds_since(t_start);
-		tp                              = Clock::now();
-		if ((e = cudaStreamSynchronize(st)))
-			return cuda_fail(e, "tridiagonal reduction");
-		ge.assign(ng, GroupReduction {});
-		for (size_t g = 0; g < ng; ++g) {
-			const size_t n = d->group_size[g];
-			if (n == 0)
-				continue;
-			GroupReduction& r = ge[g];
-			const double *  gd = h_tri + eoff[g], *go = gd + N1, *gv = go + N1;
-			r.d.assign(gd, gd + n);
-			r.off.assign(go, go + std::max<size_t>(n - 1, 1));
-			r.shift = h_shift[g];
-			double top = -INFINITY; // bisection may leave equal values an ulp out of order
-			for (size_t i = 0; i < n; ++i) {
-				if (!std::isfinite(gd[i]) || !std::isfinite(go[i]) || !std::isfinite(gv[i]))
-					return not_converged(g);
-				top                                 = std::max(top, gv[i]);
-				eigenvalues[eoff[g] + (long long)i] = r.shift ? std::ldexp(top, -r.shift) : top;
-				if (r.shift)
-					r.scaled_values.push_back(top);
+		const bool ok = group_eigenvalues(hg.size(), hn.data(), ga.data(), gw.data(), red, hw);
+		for (size_t q = 0; q < hg.size(); ++q) {
+			if (!ok && !red[q].ok) {
+				cudaStreamSynchronize(st); // the copies to this thread's buffers
+				return not_converged(hg[q]);
 			}
+			ge[hg[q]] = std::move(red[q]);
 		}
-	} else {
-		double* h_rho = pinned<double>(0, rho_elems);
-		if (!h_rho)
-			return fail(DMRGPP_OOM, "page-locked host buffer for the density matrices");
-		if ((e = cudaGetLastError())
-		    || (e = cudaMemcpyAsync(h_rho, rho, rho_elems * sizeof(double), cudaMemcpyDeviceToHost, st))
-		    || (e = cudaStreamSynchronize(st)))
-			return cuda_fail(e, "density matrices");
-		g_trunc_times[DMRGPP_TRUNC_RHO] = seconds_since(t_start);
-		tp                              = Clock::now();
-		std::vector<double*> ga(ng), gw(ng);
-		for (size_t g = 0; g < ng; ++g) {
-			ga[g] = h_rho + goff[g];
-			gw[g] = eigenvalues + eoff[g];
-		}
-		if (!group_eigenvalues(ng, d->group_size, ga.data(), gw.data(), ge, hw)) {
-			size_t g = 0;
-			while (g < ng && ge[g].ok)
-				++g;
-			return not_converged(g);
+	}
+	if ((e = cudaStreamSynchronize(st)))
+		return cuda_fail(e, "tridiagonal reduction");
+	for (const TridiagJob& j : tj) {
+		GroupReduction& r  = ge[size_t(j.group)];
+		const size_t    n  = size_t(j.n);
+		const double *  gd = h_tri + j.e_off, *go = gd + N1, *gv = go + N1;
+		r.d.assign(gd, gd + n);
+		r.off.assign(go, go + std::max<size_t>(n - 1, 1));
+		r.shift = h_shift[j.group];
+		double top = -INFINITY; // bisection may leave equal values an ulp out of order
+		for (size_t i = 0; i < n; ++i) {
+			if (!std::isfinite(gd[i]) || !std::isfinite(go[i]) || !std::isfinite(gv[i]))
+				return not_converged(size_t(j.group));
+			top                                  = std::max(top, gv[i]);
+			eigenvalues[j.e_off + (long long)i] = r.shift ? std::ldexp(top, -r.shift) : top;
+			if (r.shift)
+				r.scaled_values.push_back(top);
 		}
 	}
 
@@ -854,14 +898,10 @@ extern "C" int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, d
 		for (size_t g = 0; g < ng; ++g)
 			koff[g + 1] = koff[g] + (long long)(d->group_size[g] * kept[g]);
 		const size_t        kelems = size_t(std::max<long long>(koff[ng], 1));
-		// the host reduction's packed reflectors: every group with kept states
-		// copies its whole n x n block; the rest is never read
-		double* hv = on_device ? nullptr : pinned<double>(1, rho_elems);
 		double* zk = pinned<double>(2, kelems);
 		double* vo = pinned<double>(3, kelems);
-		if ((!on_device && !hv) || !zk || !vo)
+		if (!zk || !vo)
 			return fail(DMRGPP_OOM, "page-locked host buffers for the eigenvectors");
-		std::vector<double> bt(size_t(std::max<long long>(eoff[ng], 1)), 0.0);
 		std::vector<const double*> gwk(ng);
 		std::vector<double*>       gz(ng);
 		for (size_t g = 0; g < ng; ++g) {
@@ -869,14 +909,11 @@ extern "C" int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, d
 			gz[g]  = zk + koff[g];
 		}
 		group_eigenvectors(ng, d->group_size, kept, ge.data(), gwk.data(), gz.data(), hw);
-		if (!on_device)
-			parallel_for(ng, [&](size_t t) {
-				const size_t g = by_size[t];
-				if (kept[g] == 0)
-					return;
-				std::copy(ge[g].hv.begin(), ge[g].hv.end(), hv + goff[g]);
-				std::copy(ge[g].beta.begin(), ge[g].beta.end(), bt.begin() + eoff[g]);
-			});
+		// the host's reflectors take the place of their density matrices, as the
+		// device's have (h_rho's buffer is free again)
+		parallel_for(hg.size(), [&](size_t q) {
+			std::copy(ge[hg[q]].hv.begin(), ge[hg[q]].hv.end(), h_rho + hoff[q]);
+		});
 		g_trunc_times[DMRGPP_TRUNC_VECTORS_HOST] = seconds_since(tp);
 		tp                                       = Clock::now();
 		std::vector<ColumnJob> cj;
@@ -884,10 +921,10 @@ extern "C" int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, d
 			for (int j = 0; j < int(kept[g]); ++j)
 				cj.push_back({ koff[g], koff[g], goff[g], eoff[g], int(d->group_size[g]), j, j, 0 });
 		if (!cj.empty()) {
-			double *   z = nullptr, *v = nullptr, *d_hv = nullptr, *d_bt = nullptr;
+			double *   z = nullptr, *v = nullptr;
 			ColumnJob* d_cj = nullptr;
 			struct FreeV {
-				double**    a[4];
+				double**    a[2];
 				ColumnJob** j;
 				~FreeV()
 				{
@@ -895,23 +932,25 @@ extern "C" int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, d
 						dev_free(*p);
 					dev_free(*j);
 				}
-			} freev { { &z, &v, &d_hv, &d_bt }, &d_cj };
+			} freev { { &z, &v }, &d_cj };
 			if ((e = dev_malloc(&z, kelems * sizeof(double))) || (e = dev_malloc(&v, kelems * sizeof(double)))
 			    || (e = dev_malloc(&d_cj, cj.size() * sizeof(ColumnJob))))
 				return cuda_fail(e, "eigenvector allocation");
-			// the device reduction left its reflectors in rho's storage
-			if (!on_device
-			    && ((e = dev_malloc(&d_hv, rho_elems * sizeof(double))) || (e = dev_malloc(&d_bt, bt.size() * sizeof(double)))
-			        || (e = cudaMemcpyAsync(d_hv, hv, rho_elems * sizeof(double), cudaMemcpyHostToDevice, st))
-			        || (e = cudaMemcpyAsync(d_bt, bt.data(), bt.size() * sizeof(double), cudaMemcpyHostToDevice, st))))
-				return cuda_fail(e, "eigenvector set-up");
-			const double* refl = on_device ? rho : d_hv;
-			const double* rbet = on_device ? tri + 3 * std::max<size_t>(N, 1) : d_bt;
+			for (size_t q = 0; q < hg.size(); ++q) {
+				const GroupReduction& r = ge[hg[q]];
+				if (kept[hg[q]] == 0 || r.beta.empty())
+					continue;
+				if ((e = cudaMemcpyAsync(rho + goff[hg[q]], h_rho + hoff[q], size_t(hoff[q + 1] - hoff[q]) * sizeof(double),
+				                         cudaMemcpyHostToDevice, st))
+				    || (e = cudaMemcpyAsync(dbeta + eoff[hg[q]], r.beta.data(), r.beta.size() * sizeof(double),
+				                            cudaMemcpyHostToDevice, st)))
+					return cuda_fail(e, "reflector upload");
+			}
 			if ((e = cudaMemcpyAsync(z, zk, kelems * sizeof(double), cudaMemcpyHostToDevice, st))
 			    || (e = cudaMemcpyAsync(d_cj, cj.data(), cj.size() * sizeof(ColumnJob), cudaMemcpyHostToDevice, st)))
 				return cuda_fail(e, "eigenvector set-up");
 			const int cgrid = int(std::min<size_t>((cj.size() + 7) / 8, 148 * 8));
-			k_back_transform<<<std::max(cgrid, 1), 256, 0, st>>>(z, v, refl, rbet, d_cj, int(cj.size()));
+			k_back_transform<<<std::max(cgrid, 1), 256, 0, st>>>(z, v, rho, dbeta, d_cj, int(cj.size()));
 			if ((e = cudaGetLastError())
 			    || (e = cudaMemcpyAsync(vo, v, size_t(koff[ng]) * sizeof(double), cudaMemcpyDeviceToHost, st))
 			    || (e = cudaStreamSynchronize(st)))

@@ -84,3 +84,11 @@ def test_group_above_the_device_limit(cuda_lib, cuda_device):
     sizes, rights = [2049, 9], [40, 12]
     psi = np.concatenate([rng.standard_normal(n * r) for n, r in zip(sizes, rights)])
     _check(sizes, rights, psi / np.linalg.norm(psi), 20)
+
+
+def test_groups_on_both_sides_of_the_device_limit(cuda_lib, cuda_device):
+    """The device's largest group beside one for the host, and small ones."""
+    rng = np.random.default_rng(8)
+    sizes, rights = [300, 2049, 31, 2048, 1], [310, 60, 40, 70, 3]
+    psi = np.concatenate([rng.standard_normal(n * r) for n, r in zip(sizes, rights)])
+    _check(sizes, rights, psi / np.linalg.norm(psi), 200)
