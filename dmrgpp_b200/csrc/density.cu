@@ -803,15 +803,13 @@ extern "C" int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, d
 			if (v)
 				cudaEventDestroy(v);
 		}
-	} copied; // the host's density matrices are there
-	if (!hg.empty()) {
-		for (size_t q = 0; q < hg.size(); ++q)
-			if ((e = cudaMemcpyAsync(h_rho + hoff[q], rho + goff[hg[q]], size_t(hoff[q + 1] - hoff[q]) * sizeof(double),
-			                         cudaMemcpyDeviceToHost, st)))
-				return cuda_fail(e, "density matrices");
-		if ((e = cudaEventCreateWithFlags(&copied.v, cudaEventDisableTiming)) || (e = cudaEventRecord(copied.v, st)))
+	} formed; // the density matrices are there, the host's also in its buffer
+	for (size_t q = 0; q < hg.size(); ++q)
+		if ((e = cudaMemcpyAsync(h_rho + hoff[q], rho + goff[hg[q]], size_t(hoff[q + 1] - hoff[q]) * sizeof(double),
+		                         cudaMemcpyDeviceToHost, st)))
 			return cuda_fail(e, "density matrices");
-	}
+	if ((e = cudaEventCreateWithFlags(&formed.v, cudaEventDisableTiming)) || (e = cudaEventRecord(formed.v, st)))
+		return cuda_fail(e, "density matrices");
 	double *dd = tri, *doff = tri + N1, *dw = tri + 2 * N1, *dbeta = tri + 3 * N1;
 	if (!tj.empty()) {
 		k_tridiag<<<unsigned(tj.size() * kTriCluster), kTriThreads, tri_smem, st>>>(
@@ -823,12 +821,12 @@ extern "C" int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, d
 	    || (e = cudaMemcpyAsync(h_tri, tri, 3 * N1 * sizeof(double), cudaMemcpyDeviceToHost, st))
 	    || (e = cudaMemcpyAsync(h_shift, d_shift, ng * sizeof(int), cudaMemcpyDeviceToHost, st)))
 		return cuda_fail(e, "tridiagonal reduction");
+	if ((e = cudaEventSynchronize(formed.v)))
+		return cuda_fail(e, "density matrices");
 	g_trunc_times[DMRGPP_TRUNC_RHO] = seconds_since(t_start);
 	auto tp                         = Clock::now();
 	ge.assign(ng, GroupReduction {});
 	if (!hg.empty()) {
-		if ((e = cudaEventSynchronize(copied.v)))
-			return cuda_fail(e, "density matrices");
 		std::vector<GroupReduction> red;
 		std::vector<size_t>         hn;
 		std::vector<double*>        ga, gw;

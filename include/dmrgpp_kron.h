@@ -690,9 +690,10 @@ int dmrgpp_density_truncate(const dmrgpp_density_desc* d, size_t m, double toler
 
 /* Wall-clock seconds of the phases of the calling thread's last
  * dmrgpp_density_truncate (host clock, each phase waiting for its device
- * work): RHO the density matrices (device, to the host), EIGENVALUES the
- * tridiagonal reductions and eigenvalues (host cores), SELECT the ranking,
- * VECTORS_HOST the inverse iterations and packing, VECTORS_DEVICE the
+ * work): RHO the density matrices (device; of groups above 2048 states also
+ * the copy to the host), EIGENVALUES the tridiagonal reductions and
+ * eigenvalues (device; groups above 2048 states on the host cores meanwhile),
+ * SELECT the ranking, VECTORS_HOST the inverse iterations, VECTORS_DEVICE the
  * back-transformation and copy out, TOTAL the whole call.  n (<=
  * DMRGPP_TRUNC_NPHASES) values are written to t. */
 enum {

@@ -92,3 +92,18 @@ def test_groups_on_both_sides_of_the_device_limit(cuda_lib, cuda_device):
     sizes, rights = [300, 2049, 31, 2048, 1], [310, 60, 40, 70, 3]
     psi = np.concatenate([rng.standard_normal(n * r) for n, r in zip(sizes, rights)])
     _check(sizes, rights, psi / np.linalg.norm(psi), 200)
+
+
+def test_phase_times_belong_to_their_phases(cuda_lib, cuda_device):
+    """A density matrix of 16 states from 2^21 columns: its product takes one
+    CTA milliseconds, its reduction and eigenvalues a fraction of one."""
+    import torch
+    from dmrgpp_b200 import truncation
+    n, r = 16, 1 << 21
+    psi = torch.randn(n * r, dtype=torch.float64, device="cuda")
+    psi /= torch.linalg.vector_norm(psi)
+    for _ in range(2):
+        truncation.density_truncate([n], [r], np.arange(1), [n], 0, psi, 4)
+    t = truncation.truncation_profile()
+    assert t["rho"] > 2.0 * t["eigenvalues"]
+    assert sum(v for k, v in t.items() if k != "total") <= t["total"] * (1 + 1e-9)
