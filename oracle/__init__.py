@@ -39,14 +39,18 @@ _dp = ctypes.POINTER(ctypes.c_double)
 _vpp = ctypes.POINTER(ctypes.c_void_p)
 
 
+def ref_sources() -> bool:
+    """Whether the reference's sources are there to build the harness from (an
+    empty folder is none)."""
+    return os.path.isfile(os.path.join(REFERENCE_TREE, "dmrg", "Engine", "MatrixVectorKron", "BatchedGemmCpu.h"))
+
+
 def build(force: bool = False) -> None:
-    """Compile the C restatement and, when the reference tree is present,
+    """Compile the C restatement and, when the reference's sources are there,
     the reference harness."""
     if force or not os.path.exists(ORACLE_SO):
         subprocess.run(["make", "-s", "-C", HERE, "liboracle_kron.so"], check=True)
-    if os.path.isfile(os.path.join(REFERENCE_TREE, "dmrg", "Engine", "MatrixVectorKron",
-                                   "BatchedGemmCpu.h")) and (force or not os.path.exists(REF_SO)
-                                          or not os.path.exists(REF_KC_SO)):
+    if ref_sources() and (force or not os.path.exists(REF_SO) or not os.path.exists(REF_KC_SO)):
         subprocess.run(["make", "-s", "-C", HERE, "ref", "REF=" + REFERENCE_TREE], check=True)
 
 

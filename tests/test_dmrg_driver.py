@@ -7,6 +7,7 @@ import os
 
 import pytest
 
+import oracle
 from oracle import dmrg_driver as dd
 
 GOLDEN = os.path.join(os.path.dirname(__file__), "golden")
@@ -26,6 +27,8 @@ def test_hubbard_L4_exact(U):
         assert abs(e - dd.free_fermion_energy(4, 2, 2)) < 1e-12
 
 
+@pytest.mark.skipif(not oracle.ref_sources() and not oracle.ref_available(),
+                    reason="reference harness not built")
 def test_hubbard_L8_U0_reference_solver(oracle_built):
     """dmrg/CMakeLists.txt:180-181 (input2_batchedgemm): Hubbard L=8, U=0,
     half filling, -9.51754; exact free-fermion value -9.517540966..."""

@@ -68,9 +68,7 @@ def test_zero_and_missing_blocks_do_not_contribute(oracle_built):
     np.testing.assert_allclose(y, prob.dense() @ x, rtol=1e-13)
 
 
-@pytest.mark.skipif(not os.path.isdir(oracle.REFERENCE_TREE) and
-                    not os.path.exists(os.path.join(os.path.dirname(__file__), "..", "oracle",
-                                                    "_ref", "libref_kron.so")),
+@pytest.mark.skipif(not oracle.ref_sources() and not oracle.ref_available(),
                     reason="reference harness not built")
 @pytest.mark.parametrize("seed", range(3))
 def test_oracle_vs_reference_batched_gemm_cpu(oracle_built, seed):
@@ -82,9 +80,7 @@ def test_oracle_vs_reference_batched_gemm_cpu(oracle_built, seed):
     np.testing.assert_allclose(y, y_ref, rtol=1e-12, atol=1e-13)
 
 
-@pytest.mark.skipif(not os.path.isdir(oracle.REFERENCE_TREE) and
-                    not os.path.exists(os.path.join(os.path.dirname(__file__), "..", "oracle",
-                                                    "_ref", "libref_kron.so")),
+@pytest.mark.skipif(not oracle.ref_sources() and not oracle.ref_available(),
                     reason="reference harness not built")
 def test_oracle_vs_reference_on_microbench_sector(oracle_built):
     prob = sb.c2_problem()
@@ -135,8 +131,8 @@ def test_gather_index_restates_copy_in(oracle_built):
     assert sorted(idx.tolist()) == list(range(dim))
 
 
-@pytest.mark.skipif(not os.path.isdir(oracle.REFERENCE_TREE) and
-                    not os.path.exists(oracle.REF_KC_SO), reason="reference harness not built")
+@pytest.mark.skipif(not oracle.ref_sources() and not os.path.exists(oracle.REF_KC_SO),
+                    reason="reference harness not built")
 @pytest.mark.parametrize("threads", [1, 4])
 def test_reference_nonbatched_path_matches_restatement(oracle_built, threads):
     """The reference's default CPU H*x (KronConnections::doTask with
@@ -151,8 +147,8 @@ def test_reference_nonbatched_path_matches_restatement(oracle_built, threads):
         assert np.abs(y - ref).max() <= 1e-12 * np.abs(ref).max()
 
 
-@pytest.mark.skipif(not os.path.isdir(oracle.REFERENCE_TREE) and
-                    not os.path.exists(oracle.REF_KC_SO), reason="reference harness not built")
+@pytest.mark.skipif(not oracle.ref_sources() and not os.path.exists(oracle.REF_KC_SO),
+                    reason="reference harness not built")
 def test_reference_kron_methods_on_the_kronutil_test_grid(oracle_built):
     """The grid of the reference's own KronUtil test (dmrg/KronUtil/test1.cpp:
     A blocks of 1, 4, 7 rows and columns, B blocks of 1, 4, 7, 10 rows and
