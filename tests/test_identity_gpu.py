@@ -30,8 +30,8 @@ def test_identity_terms_and_ragged_tiles(cuda_lib, cuda_device, oracle_built, le
     bg.close()
 
 
-# rows around one chunk of the projections (512), odd and even; a chunk of
-# several; the largest group of columns of one step
+# rows around one chunk of the projections (512), odd and even; six blocks of
+# one chunk (several chunks a block: test_lanczos_chunks_gpu.py)
 @pytest.mark.parametrize("left,right", [([511], [1]), ([512], [1]), ([513], [1]), ([32, 33], [32, 31]), ([60], [51])])
 def test_lanczos_chunk_edges(cuda_lib, cuda_device, left, right):
     from dmrgpp_b200 import plugin
