@@ -492,32 +492,31 @@ bool validation_requested()
 
 // The FP64 configuration of a new handle (the tuner replaces it by the fastest
 // on the sector itself).  Where the lines lie, from sweeps of spin links,
-// Hubbard chains and ladders and sector groups on a B200 (us per H*x):
+// Hubbard chains and ladders and sector groups on a B200 in every
+// configuration (us per H*x):
 // * few patches, each within one fused column tile: the fused form has no
-//   dependent second pass (5 to 21 patches: 8.5 against 11.5 with two passes,
-//   12.4 against 16.5, microbench sector 27.6 against 34.8); with many small
-//   patches its units are too short (145 patches: 33 against 32), and above
-//   4e8 flops the heaviest part sets its end (6e8: 126 against 72);
+//   dependent second pass (against the best two-pass configuration: 5 patches
+//   8.3 / 10.3, 13 patches 12.4 / 13.8, 17 patches 20.6 / 22.6, microbench
+//   sector 28.6 / 30.3).  With many small patches its units are too short (57
+//   patches: 17.2 / 17.0, 129 patches: 24.7 / 16.8), with more work the
+//   heaviest part sets its end (2.7e8 flops: 54.2 / 54.0, 4.3e8: 74 / 49), and
+//   wider patches repeat the first product (162 columns: 60 / 38);
 // * small work: 32 x 32 tiles with k-chunks of 32, half as many steps in the
-//   latency-bound chains (chain of 4000 states 49.3 against 56.1 with chunks
-//   of 16); from 6e8 flops shorter chunks waste less of ragged patches
-//   (batch of 8 sectors 66.5 against 70.0) unless patches are wide (ladder of
-//   10000 states, patches to 332: 445 against 460);
+//   latency-bound chains (chain of 4000 states, 5e8 flops: 47.0 against 56.3
+//   with chunks of 16; either may win by a tenth from 3e8 to 6e8);
+// * from 6e8 flops shorter chunks waste less of ragged patches (batch of 8
+//   sectors 65.1 against 66.8, ladder of 6000 states 139 against 149, of 10000
+//   404 against 427, few wide patches 275 against 288; at worst 87.2 against
+//   86.1);
 // * 64 x 64 tiles only where the sector fills the SMs several times over with
-//   them: 1396 against 1449 at 3.6e10 flops, but 740 against 700 at 1.6e10
-//   and 2 to 4 times slower below 1e9.
+//   them: 1299 against 1332 at 3.6e10 flops, but 692 against 645 at 1.6e10
+//   and 2 to 5 times slower below 1e9.
 DefaultConfig default_config(const KronPlan& plan, long long fused_bn)
 {
-	long long widest = 0, max_l = 0;
-	for (size_t p = 0; p < plan.np; ++p) {
-		max_l  = std::max(max_l, plan.l[p]);
-		widest = std::max({ widest, plan.l[p], plan.r[p] });
-	}
+	const long long max_l = plan.l.empty() ? 0 : *std::max_element(plan.l.begin(), plan.l.end());
 	if (plan.np <= 40 && max_l <= fused_bn && plan.f_alg < 4e8)
 		return { true, 0, 1 };
-	if (plan.f_alg >= 2.5e10)
-		return { false, 2, 2 };
-	return { false, plan.f_alg >= 6e8 && widest < 320 ? 0 : 1, 2 };
+	return { false, plan.f_alg >= 2.5e10 ? 2 : plan.f_alg >= 6e8 ? 0 : 1, 2 };
 }
 
 std::string validate_persistent_schedule(const KronPlan& plan, int tile)

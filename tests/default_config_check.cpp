@@ -23,11 +23,10 @@ int main()
 		{ 41, 128, 400, 3.9e8, false, 1, 1 },     // ... and one step past each
 		{ 40, 129, 400, 3.9e8, false, 1, 1 },
 		{ 40, 128, 400, 4e8, false, 1, 1 },
-		{ 200, 300, 319, 6e8, false, 0, 0 },
-		{ 200, 300, 320, 6e8, false, 1, 1 },
-		{ 200, 300, 319, 5.9e8, false, 1, 1 },
+		{ 200, 300, 320, 6e8, false, 0, 0 },
+		{ 200, 300, 320, 5.9e8, false, 1, 1 },
 		{ 300, 500, 500, 2.5e10, false, 2, 2 },
-		{ 300, 500, 500, 2.4e10, false, 1, 1 },
+		{ 300, 500, 500, 2.4e10, false, 0, 0 },
 	};
 	int n = 0;
 	for (const Case& c : cases) {
