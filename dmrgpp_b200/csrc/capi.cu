@@ -624,13 +624,14 @@ int finish_create(dmrgpp_kron_handle h, int device, void* stream, Clock::time_po
 
 	if ((e = dmrgpp::error_word_alloc(&h->err_host, &h->err_dev)))
 		return bail(e, "error word");
-	dmrgpp::DefaultConfig dc = dmrgpp::default_config(P, dmrgpp::fused_shape(0).bn);
-	int                   clusters = 0;
-	if (dc.fused && (dmrgpp::fused_init(0, &clusters) != cudaSuccess || clusters < 1)) {
-		// no cluster of the fused form fits (a share of the SMs, say): two passes
+	const dmrgpp::FusedShape fs       = dmrgpp::fused_shape(0);
+	int                      clusters = 0;
+	if (dmrgpp::fused_init(0, &clusters) != cudaSuccess) { // (a restricted share of the SMs may hold none)
 		cudaGetLastError();
-		dc = dmrgpp::default_config(P, 0);
+		clusters = 0;
 	}
+	const dmrgpp::DefaultConfig dc
+	    = dmrgpp::default_config(h->plan, fs.bm, fs.bn, fs.cw, fs.cluster, clusters);
 	if (int rc = dmrgpp::configure_schedule(h, dc.fused ? dmrgpp::kNumTileCfgs : dc.cfg, dc.items_per_cta)) {
 		const std::string why = h->err;
 		release(h);

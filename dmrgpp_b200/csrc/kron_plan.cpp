@@ -494,13 +494,17 @@ bool validation_requested()
 // on the sector itself).  Where the lines lie, from sweeps of spin links,
 // Hubbard chains and ladders and sector groups on a B200 in every
 // configuration (us per H*x):
-// * few patches, each within one fused column tile: the fused form has no
-//   dependent second pass (against the best two-pass configuration: 5 patches
+// * the fused form has no dependent second pass, but walks a tile's units 16 of
+//   the contraction at a time (about 1.06 us a step of the busiest cluster, 6.5
+//   us besides).  It takes a sector of few patches of one column tile whose
+//   parts all run at once (against the best two-pass configuration: 5 patches
 //   8.3 / 10.3, 13 patches 12.4 / 13.8, 17 patches 20.6 / 22.6, microbench
-//   sector 28.6 / 30.3).  With many small patches its units are too short (57
-//   patches: 17.2 / 17.0, 129 patches: 24.7 / 16.8), with more work the
-//   heaviest part sets its end (2.7e8 flops: 54.2 / 54.0, 4.3e8: 74 / 49), and
-//   wider patches repeat the first product (162 columns: 60 / 38);
+//   sector 28.6 / 30.3).  A second round of clusters doubles its time (20
+//   patches of 16 x 128: 36 / 19, of 100 x 100: 72 / 43, 30 of 3 x 300: 173 /
+//   52), long right groups make its steps many (two patches of 4 x 200: 16.5 /
+//   18.6, of 4 x 300: 22.7 / 20.7, one of 1 x 1000: 68 / 49), wider left ones
+//   repeat the first product (162 columns: 60 / 38), and it gains nothing from
+//   57 patches (17.2 / 17.0) or 2.7e8 flops (54.2 / 54.0) on;
 // * small work: 32 x 32 tiles with k-chunks of 32, half as many steps in the
 //   latency-bound chains (chain of 4000 states, 5e8 flops: 47.0 against 56.3
 //   with chunks of 16; either may win by a tenth from 3e8 to 6e8);
@@ -511,11 +515,18 @@ bool validation_requested()
 // * 64 x 64 tiles only where the sector fills the SMs several times over with
 //   them: 1299 against 1332 at 3.6e10 flops, but 692 against 645 at 1.6e10
 //   and 2 to 5 times slower below 1e9.
-DefaultConfig default_config(const KronPlan& plan, long long fused_bn)
+DefaultConfig default_config(KronPlan& plan, int bm, int bn, int cw, int cluster, int clusters)
 {
-	const long long max_l = plan.l.empty() ? 0 : *std::max_element(plan.l.begin(), plan.l.end());
-	if (plan.np <= 40 && max_l <= fused_bn && plan.f_alg < 4e8)
-		return { true, 0, 1 };
+	long long max_l = 0, max_r = 0;
+	for (size_t p = 0; p < plan.np; ++p) {
+		max_l = std::max(max_l, plan.l[p]);
+		max_r = std::max(max_r, plan.r[p]);
+	}
+	if (clusters > 0 && plan.np <= 40 && max_l <= bn && max_r <= 256 && plan.f_alg < 4e8) {
+		build_fused_schedule(plan, bm, bn, cw, cluster, 1, clusters * cluster);
+		if (plan.fitems.size() <= size_t(clusters) * size_t(cluster))
+			return { true, 0, 1 };
+	}
 	return { false, plan.f_alg >= 2.5e10 ? 2 : plan.f_alg >= 6e8 ? 0 : 1, 2 };
 }
 

@@ -457,16 +457,6 @@ constexpr int kMaxItemSegs = 32;
 // k boundary) of about the length that makes items_per_cta of them per CTA.
 void build_persistent_schedule(KronPlan& plan, int bk, int grid, int items_per_cta = 2);
 
-// The FP64 configuration of a new handle: the fused form or a two-pass
-// configuration (kron_persistent.cuh), and its items_per_cta.  fused_bn: the
-// columns of the fused form's output tile, 0 where that form cannot run.
-struct DefaultConfig {
-	bool fused;
-	int  cfg;
-	int  items_per_cta;
-};
-DefaultConfig default_config(const KronPlan& plan, long long fused_bn);
-
 // Checks the persistent work list against the buffers before a launch (the
 // host-side bounds check of the debug mode, DMRGPP_VALIDATE=1): for every
 // item, with tile x tile output tiles, the first and last element of each
@@ -507,5 +497,17 @@ bool validation_requested();
 // (optional, np entries) gives each output patch's sector for group handles.
 void build_fused_schedule(KronPlan& plan, int bm, int bn, int cw, int cluster, int rounds,
                           int ctas, const std::vector<int>* sector_of_patch = nullptr);
+
+// The FP64 configuration of a new handle: the fused form or a two-pass
+// configuration (kron_persistent.cuh), and its items_per_cta.  bm, bn, cw,
+// cluster: the fused form's shape; clusters: how many of its clusters are
+// resident at once, 0 where that form cannot run.  (Builds plan.fitems and
+// plan.funits where it considers the fused form.)
+struct DefaultConfig {
+	bool fused;
+	int  cfg;
+	int  items_per_cta;
+};
+DefaultConfig default_config(KronPlan& plan, int bm, int bn, int cw, int cluster, int clusters);
 
 } // namespace dmrgpp
