@@ -110,7 +110,7 @@ __device__ __forceinline__ double block_sum_all(double v, double* red)
 // formed by every CTA for itself.  All groups run side by side: the launch
 // lasts as long as the largest group's n steps of a few memory latencies each
 // (the host cores took 10.6 ms for 241 groups of up to 532 states with their
-// eigenvalues, this kernel 3.8).
+// eigenvalues, this kernel 3.9).
 __global__ void __cluster_dims__(kTriCluster, 1, 1) __launch_bounds__(kTriThreads)
 k_tridiag(double* __restrict__ rho, double* __restrict__ work, const TridiagJob* __restrict__ jobs, double* d,
           double* off, double* beta, int* shift, int vec)

@@ -76,12 +76,21 @@ std::string build_wft_plan(const dmrgpp_wft_desc& d, WftPlan& plan, std::vector<
 	}
 	if (plan.x_start.back() > (long long)INT_MAX * 64 || plan.y_start.back() > (long long)INT_MAX * 64)
 		return "sector too large";
-	// 64 x 64 tiles where they fill the SMs with four CTAs each; smaller layouts
-	// are latency-bound and want more, smaller tiles
+	// 64 x 64 tiles where the outputs are worth 512 of them (us for both passes,
+	// 64 against 32: ladder of 16000 states, worth 822, 183 / 195; 13000 states,
+	// 553, 116 / 121; but 12000 states, 472, 108 / 98 and 10000 states, 332, 74 /
+	// 64), or 250 where they are nearly full (a patch of 1500 x 1500 463 / 527,
+	// eight of 500 x 500 169 / 185; at 250 the two take the same).  Smaller and more
+	// ragged layouts are latency-bound and want more, smaller tiles (30 patches of
+	// 200 x 200 74 / 62, ladder of 8000 states 41 / 33).
 	long long tiles64 = 0;
-	for (size_t q = 0; q < d.np_out; ++q)
+	double    area    = 0.0; // in tiles
+	for (size_t q = 0; q < d.np_out; ++q) {
 		tiles64 += ((plan.l_out[q] + 63) / 64) * ((plan.r_out[q] + 63) / 64);
-	plan.bm = plan.bn = maxs > 192 && tiles64 >= 4 * 148 ? 64 : 32;
+		area += double(plan.l_out[q]) * double(plan.r_out[q]) / 4096.0;
+	}
+	const bool large = area >= 512.0 || (tiles64 >= 250 && area >= 0.85 * double(tiles64));
+	plan.bm = plan.bn = maxs > 192 && large ? 64 : 32;
 
 	// packed blocks and the intermediate T
 	plan.wr_off.assign(d.np_out, 0);

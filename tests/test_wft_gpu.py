@@ -38,6 +38,22 @@ def rel_err(y, ref):
     return float(np.abs(y - ref).max() / max(np.abs(ref).max(), 1e-300))
 
 
+# uniform patches on both sides of the tile choice: 64 x 64 tiles nearly full
+# (256 of them, and 289 with ragged edges), too few, and too ragged
+@pytest.mark.parametrize("sizes", [[512] * 4, [1030], [500] * 3, [200] * 30])
+def test_uniform_layouts_match_oracle(cuda_lib, cuda_device, sizes):
+    from dmrgpp_b200.wft import WaveFunctionTransform
+    from oracle import wft_oracle
+    rng = np.random.default_rng(len(sizes))
+    n = np.array(sizes)
+    lay = (n, n - 1, n - 2, n, list(range(len(sizes))))
+    WL, WR = _blocks(rng, *lay, 0, 0)
+    w = WaveFunctionTransform(*lay, WL, WR)
+    x = rng.standard_normal(w.dim_in)
+    assert rel_err(w(x), wft_oracle.transform(x, *lay, WL, WR)) < RTOL
+    w.close()
+
+
 @pytest.mark.parametrize("seed,npi,npo,maxs,tl,tr", [
     (0, 1, 1, 1, 0, 0), (1, 4, 5, 20, 0, 0), (2, 6, 6, 70, 1, 0), (3, 5, 7, 33, 0, 1),
     (4, 3, 3, 200, 1, 1), (5, 10, 12, 50, 0, 0), (6, 2, 4, 130, 1, 1)])
