@@ -379,15 +379,22 @@ __device__ __forceinline__ void store_partial(const TcArgs& a, const GemmTile& t
 }
 
 // after every part of split tile t wrote its slot: sum the slots in part
-// order (deterministic) and write y
+// order (deterministic) and write y.  A tile of few rows leaves warps without
+// any: they take column chunks of the other rows, whose loads are one memory
+// latency per part and chunk (pass 2 of four patches of 1000 x 16 states 46.0 ->
+// 34.3 us, of 20 of 300 x 30 33.2 -> 24.1)
 template <int BN>
-__device__ __forceinline__ void reduce_split(const TcArgs& a, const GemmTile& t, int row, int vn)
+__device__ __forceinline__ void reduce_split(const TcArgs& a, const GemmTile& t, int thread, int vn)
 {
+	const int rgroups = min(4, (t.M - t.m0 + 31) >> 5); // groups of 32 rows
+	const int cgroups = 4 / rgroups;
+	const int rg = (thread >> 5) % rgroups, cg = (thread >> 5) / rgroups;
+	const int row  = rg * 32 + (thread & 31);
 	const int grow = t.m0 + row;
-	if (grow >= t.M)
+	if (grow >= t.M || cg >= cgroups)
 		return;
 	double* y = (a.io ? a.io->y : a.Cd) + t.c_off;
-	for (int c0 = 0; c0 < vn; c0 += 32) {
+	for (int c0 = 32 * cg; c0 < vn; c0 += 32 * cgroups) {
 		float s[32];
 #pragma unroll
 		for (int i = 0; i < 32; ++i)
