@@ -173,8 +173,9 @@ int dmrgpp_kron_synchronize(dmrgpp_kron_handle h);
  * first pipeline stage of one CTA of pass 1 is never filled, so the MMA
  * thread's mbarrier wait runs out (about 0.5 s), the CTA drains its copies,
  * frees its tensor memory and exits.  The apply then reports DMRGPP_TIMEOUT
- * and the handle stays usable.  Used to test failure detection without
- * faulting the GPU. */
+ * and the handle stays usable.  A handle on the fused form, which has no such
+ * wait, runs the two-pass form until on = 0.  Used to test failure detection
+ * without faulting the GPU. */
 int dmrgpp_kron_test_stall_dependency(dmrgpp_kron_handle h, int on);
 
 /* The diagonal of the sector's H (patch order) into diag (device pointer). */
@@ -279,8 +280,9 @@ const char* dmrgpp_kron_noalloc_last_error(void);
  * set of fixed constants, BatchedGemmKokkos.h:110-130) ----
  * Tile configurations of the H*x kernel.  Two-pass persistent form:
  * 0: 32x32 tiles, k-chunk 16; 1: 32x32, k32; 2: 64x64, k16; 3: 64x64, k32;
- * 4: 32x32, k32, deeper pipeline; 5: 32x32, k64; items_per_cta: pass-2
- * work items per resident CTA below which output tiles are split along K.
+ * 4: 32x32, k32, deeper pipeline; 5: 32x32, k64; items_per_cta: about how
+ * many pass-2 work items per resident CTA the output tiles are cut into
+ * along K.
  * Fused form (both passes of an output tile in one CTA, parts of a tile
  * summed inside a thread-block cluster; for sectors of small patches):
  * 6: 32x128 output tiles, 64-column units, clusters of 8; 7: the same with
